@@ -27,7 +27,7 @@ SOURCES = ["api.cu", "bank.cu", "search.cu", "search_plane_lo.cu", "search_plane
            "search_fund_lo.cu", "search_fund_hi.cu", "tune.cu", "whiten.cu", "compat.cu",
            "server.cu", "sift.cu", "optimize.cu", "dedisperse.cu",
            "filterbank.cu", "compat_cxx.cu", "search_step.cu", "rfft.cu", "search_mixed5.cu",
-           "search_mixed6.cu", "search_mixed7.cu", "search_mixed_prep.cu"]
+           "search_mixed6.cu", "search_mixed7.cu", "search_mixed_prep.cu", "refine.cu"]
 EXTRA = {"bank.cu": ["-fmad=false"], "compat.cu": ["-Xcompiler", "-ffp-contract=off"],
          "dedisperse.cu": ["-Xcompiler", "-ffp-contract=off"]}
 HEADERS = ["accel_common.cuh", "accel_internal.h", "context.h", "fft_smem.cuh", "search_kernels.cuh",

@@ -255,6 +255,70 @@ __device__ __forceinline__ uint32_t block_select_u32(const uint32_t* keys, int n
     }
     return prefix;
 }
+
+// Exact k-th smallest (0-based) of keys the CTA's threads hold themselves:
+// each(f) calls f(key) for every key of the calling thread.  Three radix
+// passes (11, 11 and 10 bits) over a shared histogram of 2048 counters
+// (hist, 16-byte aligned); scratch: 40 ints of shared memory.  All NT
+// threads (a multiple of 32 up to 1024) call it; the result is the same in
+// every thread, and hist may be reused on return.
+//
+// Positive floats spread over a few dozen of the first pass's bins (8
+// exponent and 3 mantissa bits), so plain shared atomics meet few
+// collisions and one pass leaves about 1/30 of the keys; keys come from
+// registers or global memory.
+constexpr int kSelectBins = 2048;
+template <int NT, class Each>
+__device__ __forceinline__ uint32_t block_rank_select(Each each, int k, uint32_t* hist, int* scratch) {
+    static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t prefix = 0, mask = 0;
+#pragma unroll
+    for (int pass = 0; pass < 3; pass++) {
+        constexpr int kBits[3] = {11, 11, 10}, kShift[3] = {21, 10, 0};
+        const int shift = kShift[pass], bins = 1 << kBits[pass];
+        for (int i = tid; i < kSelectBins / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        each([&](uint32_t key) {
+            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & (uint32_t)(bins - 1)], 1u);
+        });
+        __syncthreads();
+        // bins [tid PER, tid PER + PER) of every thread, their sums scanned
+        // over the warp and, through scratch, over the CTA
+        constexpr int PER = kSelectBins / NT;
+        uint32_t sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; j++) sum += hist[tid * PER + j];
+        int incl = (int)sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) scratch[2 + warp] = incl;
+        __syncthreads();
+        int excl = incl - (int)sum;
+        for (int w = 0; w < warp; w++) excl += scratch[2 + w];
+        if (k >= excl && k < excl + (int)sum) {  // exactly one thread
+            int c = excl, d = 0;
+            for (int j = 0; j < PER; j++) {
+                const int h = (int)hist[tid * PER + j];
+                if (k >= c && k < c + h) {
+                    d = tid * PER + j;
+                    scratch[1] = k - c;
+                }
+                c += h;
+            }
+            scratch[0] = d;
+        }
+        __syncthreads();
+        prefix |= (uint32_t)scratch[0] << shift;
+        mask |= (uint32_t)(bins - 1) << shift;
+        k = scratch[1];
+        __syncthreads();
+    }
+    return prefix;
+}
 #endif  // __CUDACC__
 
 }  // namespace accel

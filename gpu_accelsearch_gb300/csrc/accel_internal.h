@@ -190,33 +190,53 @@ inline int carveout_for(const void* kernel, int threads, size_t dyn_smem) {
     return 100;
 }
 
-// Candidate refinement (k_optimize in bank.cu): one CTA per candidate.
+// Candidate refinement (refine.cu): a cluster of CTAs per candidate.
+constexpr int kRefineNodes = 64;  // nodes of a panel of the integration rule
+constexpr int kRefineValues = 8;  // double2 kept per node between grid levels
 struct OptCand {
     double r, z;            // fundamental-plane frequency and f-dot of the candidate
     int numharm;            // harmonics k r / numharm, k = 1..numharm, are summed
     int trial;
     long long lobin[kMaxHarm];  // harmonic k's segment in the candidate's step:
     int numdata[kMaxHarm];      // its median sets the power normalisation
+    int panels[kMaxHarm];       // panels of harmonic k's integration rule
+    long long scratch_off;      // first of its nodes in the scratch buffer
 };
 struct OptOut {
     double r, z, power;     // refined position and summed power
     float harm[kMaxHarm];   // power of harmonic k at the refined position
 };
-struct OptArgs {
+struct RefineArgs {
     const float2* const* spec;   // [ntrials] whitened spectra (device)
     const long long* numbins;    // [ntrials]
     const OptCand* in;
     OptOut* out;
+    double* norm2;               // [n][kMaxHarm] squared power normalisations
+    double2* scratch;            // kRefineValues per node of every candidate
     int n;
+    int maxharm;                 // largest numharm
     int refine;                  // 0: evaluate at the given position only
-    int maxdata;                 // largest numdata (shared-memory keys)
     int exact_rsqrt;
+    int maxdata;                 // largest numdata (keys of the direct form)
 };
+// Positive nodes (largest first) and weights of the rule, a kernel argument.
+struct RefineNodes {
+    double x[kRefineNodes / 2], w[kRefineNodes / 2];
+};
+int refine_panels(double z, double zreach);
+// Widest window (panels) the node rule takes; a call with a wider one runs
+// the direct form, whose work grows with the width and not its square.
+// Measured on one candidate of one harmonic, node rule against direct: z =
+// 200 0.25 / 2.9 ms, 1000 1.4 / 13, 3000 9.7 / 39, 5000 26 / 64 (217
+// panels); the lines meet near z = 12000 and the limit is z = 8900, above
+// every f-dot a bank of 16384-point segments can hold.
+constexpr int kRefineMaxPanels = 384;
 
 // ---- launchers (return 0 or -1 after a launch error) ----
 int launch_fund_sum(const FundArgs& a, int nseg, const float2* tw, cudaStream_t st);
 int launch_twiddles(float2* tw, cudaStream_t st);
-int launch_optimize(const OptArgs& a, cudaStream_t st);
+int launch_refine(const RefineArgs& a, cudaStream_t st);
+int launch_refine_direct(const RefineArgs& a, cudaStream_t st);
 int launch_bank_build(const BankHarmDev* hd_dev, const BankHarmDev* hd_host, int nh, int ntpl,
                       float2* resp, int rstride, bool fp16, cudaStream_t st);
 int launch_prep(int M, const PrepArgs& a, int nseg, const float2* tw, cudaStream_t st);

@@ -1058,6 +1058,8 @@ void free_ctx(accel_ctx* c) {
     cudaFree(c->d_ncand);
     cudaFreeHost(c->h_ncand);
     cudaFreeHost(c->h_raw);
+    cudaFree(c->opt_dev);
+    cudaFreeHost(c->opt_host);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }

@@ -310,21 +310,11 @@ int launch_bank_build(const BankHarmDev* hd_dev, const BankHarmDev* hd_host, int
     return 0;
 }
 
-
 // --------------------------------------------------------------------------
-// Candidate refinement (the reference's optimizeCandidates stub,
-// bpd_candidates.cu:24-27).
-//
-// The power the plane kernels compute at fundamental-plane position
-// (r, z) is |sum_j X[j] conj(F(r - j - z/2; z))|^2 over the 2 hw(z) bins
-// j in [ceil(r - hw), ceil(r + hw)), where F is the response that
-// generate_z_response samples (bpd_subharmonics.cu:146-226; its loop
-// variable is the argument x) and X the whitened spectrum: the planes are
-// this expression on the grid r = rlo + i/2, z even.  Here it is evaluated
-// at any (r, z), for every harmonic k r / H, k z / H (k = 1..H) of a
-// candidate, and the summed power is maximised on three nested 5 x 5 grids
-// (steps 1/4, 1/16, 1/64 in r and 1, 1/4, 1/16 in z around the best point
-// so far).
+// Candidate refinement with the responses evaluated directly, bin by bin:
+// the form for windows so wide that refine.cu's node rule, whose work grows
+// with the square of the width, is no longer the cheaper one
+// (kRefineMaxPanels in refine.cu).  Definitions as there.
 // F(x; z), evaluated directly (the reference's small-offset series
 // corrections are expansions of the same function).
 __device__ double2 response_at(double x, double z) {
@@ -376,7 +366,7 @@ __device__ double warp_power(const float2* __restrict__ X, long long nb, double 
 
 constexpr int kOptWarps = 4;
 
-__global__ void __launch_bounds__(32 * kOptWarps) k_optimize(const OptArgs a) {
+__global__ void __launch_bounds__(32 * kOptWarps) k_refine_direct(const RefineArgs a) {
     extern __shared__ uint32_t okeys[];  // a.maxdata keys
     const int ci = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -460,13 +450,13 @@ __global__ void __launch_bounds__(32 * kOptWarps) k_optimize(const OptArgs a) {
     }
 }
 
-int launch_optimize(const OptArgs& a, cudaStream_t st) {
+int launch_refine_direct(const RefineArgs& a, cudaStream_t st) {
     if (a.n <= 0) return 0;
     const size_t smem = sizeof(uint32_t) * (size_t)a.maxdata;
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_optimize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        cudaFuncSetAttribute(k_refine_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
-    k_optimize<<<a.n, 32 * kOptWarps, smem, st>>>(a);
+    k_refine_direct<<<a.n, 32 * kOptWarps, smem, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -122,6 +122,11 @@ struct accel_ctx {
     R2CEngine r2c;  // the trials' real-to-complex transforms
     std::vector<TrialBuf> trials;
 
+    // workspace of accel_optimize_candidates (grown, kept between calls)
+    void* opt_dev = nullptr;
+    void* opt_host = nullptr;               // pinned staging of its inputs and outputs
+    size_t opt_dev_cap = 0, opt_host_cap = 0;
+
     std::vector<accel_candidate> results;
     unsigned long long last_raw = 0;
 

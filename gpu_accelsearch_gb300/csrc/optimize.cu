@@ -1,7 +1,8 @@
 // optimize.cu -- host side of candidate refinement and properties
-// (accel_optimize_candidates; the kernel is k_optimize in bank.cu).
+// (accel_optimize_candidates; the kernels are in refine.cu).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <vector>
 
@@ -30,7 +31,8 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
     int rc = ensure_device(c);
     if (rc) return rc;
     std::vector<OptCand> cand((size_t)n);
-    int maxdata = 1;
+    const double zreach = refine ? 2.63 : 0.0;  // how far the grids reach in z
+    int maxharm = 1, maxdata = 1, maxpanels = 0;
     for (long long i = 0; i < n; i++) {
         const accel_candidate& x = in[i];
         if (x.trial < 0 || x.trial >= ntrials || x.numharm < 1 || x.numharm > c->nh ||
@@ -41,6 +43,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         o.z = x.z;
         o.numharm = x.numharm;
         o.trial = x.trial;
+        maxharm = std::max(maxharm, x.numharm);
         // harmonic k of H is the bank's harmonic p/q = k/H in lowest terms;
         // its segment in the candidate's step is the search's (A6/A7)
         const long long startr = rlo[x.trial] + (long long)x.step * (c->uselen / 2);
@@ -53,46 +56,92 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
             o.lobin[k - 1] = sh.lobin;
             o.numdata[k - 1] = std::min(sh.numdata, c->hp[h].M);
             maxdata = std::max(maxdata, o.numdata[k - 1]);
+            o.panels[k - 1] = refine_panels(x.z * k / x.numharm, zreach * k / x.numharm);
+            maxpanels = std::max(maxpanels, o.panels[k - 1]);
         }
     }
     if (n == 0) return ACCEL_OK;
-    const float2** d_spec = nullptr;
-    long long* d_nb = nullptr;
-    OptCand* d_in = nullptr;
-    OptOut* d_out = nullptr;
-    std::vector<OptOut> res((size_t)n);
-    cudaError_t e = cudaMalloc(&d_spec, sizeof(float2*) * ntrials);
-    if (e == cudaSuccess) e = cudaMalloc(&d_nb, sizeof(long long) * ntrials);
-    if (e == cudaSuccess) e = cudaMalloc(&d_in, sizeof(OptCand) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&d_out, sizeof(OptOut) * n);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_spec, wspec, sizeof(float2*) * ntrials, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_nb, numbins, sizeof(long long) * ntrials, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_in, cand.data(), sizeof(OptCand) * n, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) {
-        OptArgs a{};
-        a.spec = d_spec;
-        a.numbins = d_nb;
-        a.in = d_in;
-        a.out = d_out;
-        a.n = (int)n;
-        a.refine = refine != 0;
-        a.maxdata = maxdata;
-        a.exact_rsqrt = c->cfg.exact_rsqrt;
-        if (launch_optimize(a, c->stream) != 0) e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaGetLastError();
+    // launches of at most kOptBatch candidates and kOptNodes nodes, from one
+    // workspace kept by the context: spectra table, candidates, results,
+    // norms and node values
+    constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 21;
+    const bool direct = maxpanels > kRefineMaxPanels;
+    long long most = 0, most_nodes = 0;
+    std::vector<long long> ends;  // end of each launch's candidates
+    for (long long i = 0; i < n;) {
+        long long nodes = 0, j = i;
+        for (; j < n && j - i < kOptBatch; j++) {
+            long long own = 0;
+            for (int k = 0; k < cand[j].numharm && !direct; k++) own += (long long)cand[j].panels[k] * kRefineNodes;
+            if (j > i && nodes + own > kOptNodes) break;
+            cand[j].scratch_off = nodes;
+            nodes += own;
+        }
+        most = std::max(most, j - i);
+        most_nodes = std::max(most_nodes, nodes);
+        ends.push_back(j);
+        i = j;
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(res.data(), d_out, sizeof(OptOut) * n, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_spec);
-    cudaFree(d_nb);
-    cudaFree(d_in);
-    cudaFree(d_out);
-    if (e != cudaSuccess)
-        return set_error(ACCEL_ERR_CUDA, "accel_optimize_candidates: %s", cudaGetErrorString(e));
+    auto pad = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t off_nb = pad(sizeof(float2*) * ntrials), off_in = off_nb + pad(sizeof(long long) * ntrials),
+                 off_out = off_in + pad(sizeof(OptCand) * most), off_norm = off_out + pad(sizeof(OptOut) * most),
+                 off_s = off_norm + pad(sizeof(double) * kMaxHarm * most),
+                 dev_bytes = off_s + sizeof(double2) * kRefineValues * most_nodes, host_bytes = off_norm;
+    cudaError_t e = cudaSuccess;
+    if (dev_bytes > c->opt_dev_cap) {
+        cudaFree(c->opt_dev);
+        c->opt_dev = nullptr;
+        c->opt_dev_cap = 0;
+        e = cudaMalloc(&c->opt_dev, dev_bytes);
+        if (e == cudaSuccess) c->opt_dev_cap = dev_bytes;
+    }
+    if (e == cudaSuccess && host_bytes > c->opt_host_cap) {
+        cudaFreeHost(c->opt_host);
+        c->opt_host = nullptr;
+        c->opt_host_cap = 0;
+        e = cudaMallocHost(&c->opt_host, host_bytes);
+        if (e == cudaSuccess) c->opt_host_cap = host_bytes;
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return set_error(ACCEL_ERR_NOMEM, "accel_optimize_candidates: %s", cudaGetErrorString(e));
+    }
+    char* dev = static_cast<char*>(c->opt_dev);
+    char* host = static_cast<char*>(c->opt_host);
+    std::vector<OptOut> res((size_t)n);
+    long long i0 = 0;
+    for (long long i1 : ends) {
+        const long long m = i1 - i0;
+        std::memcpy(host, wspec, sizeof(float2*) * ntrials);
+        std::memcpy(host + off_nb, numbins, sizeof(long long) * ntrials);
+        std::memcpy(host + off_in, cand.data() + i0, sizeof(OptCand) * m);
+        e = cudaMemcpyAsync(dev, host, off_in + sizeof(OptCand) * m, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess) {
+            RefineArgs a{};
+            a.spec = reinterpret_cast<const float2* const*>(dev);
+            a.numbins = reinterpret_cast<const long long*>(dev + off_nb);
+            a.in = reinterpret_cast<const OptCand*>(dev + off_in);
+            a.out = reinterpret_cast<OptOut*>(dev + off_out);
+            a.norm2 = reinterpret_cast<double*>(dev + off_norm);
+            a.scratch = reinterpret_cast<double2*>(dev + off_s);
+            a.n = (int)m;
+            a.maxharm = maxharm;
+            a.refine = refine != 0;
+            a.exact_rsqrt = c->cfg.exact_rsqrt;
+            a.maxdata = maxdata;
+            if ((direct ? launch_refine_direct(a, c->stream) : launch_refine(a, c->stream)) != 0) {
+                e = cudaGetLastError();
+                if (e == cudaSuccess) e = cudaErrorUnknown;
+            }
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(host + off_out, dev + off_out, sizeof(OptOut) * m, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e != cudaSuccess)
+            return set_error(ACCEL_ERR_CUDA, "accel_optimize_candidates: %s", cudaGetErrorString(e));
+        std::memcpy(res.data() + i0, host + off_out, sizeof(OptOut) * m);
+        i0 = i1;
+    }
     for (long long i = 0; i < n; i++) {
         const OptOut& o = res[i];
         accel_optimized& y = out[i];
