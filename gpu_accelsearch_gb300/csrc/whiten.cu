@@ -79,133 +79,160 @@ __global__ void __launch_bounds__(256) k_whiten_scale(const int* __restrict__ bs
     }
 }
 
-// Warp-per-block forms of the two kernels for blocks of at most
-// kWarpBlockMax bins (the reference's widths are at most 200): eight
-// whitening blocks per CTA, no CTA-wide barriers.
+// Forms of the two kernels for blocks of at most kWarpBlockMax bins (the
+// reference's widths are at most 200): a warp per block or range, eight
+// warps per CTA, no keys or histograms in shared memory.
+//
+// Both are one pass over the spectrum (8 and 16 bytes per bin) and should be
+// bound by memory.  The first form was not: a digit histogram per warp in
+// shared memory (match_any and atomics for every key), and one
+// double-precision division per warp -- all 32 lanes of it, at 1/64 of the
+// single-precision rate -- for every level and slope.  Now the median is a
+// bitwise search over keys in registers (counts by redux.sync, stopped when
+// one key is left in the interval) and levels and slopes are computed by one
+// lane per range.  2^21 bins, GB300: medians 55 -> 17 us, scaling 31 -> 13 us
+// (cold cache).
 constexpr int kWarpBlockMax = 1024;
 constexpr int kWarpsPerCta = 8;
+constexpr int kScaleRanges = 32;  // write ranges per CTA of the scaling kernel
 
-// Exact rank-k key of keys[0..n) by an 8-bit radix select within one warp
-// (hist: 256 ints of this warp's shared memory).
-__device__ __forceinline__ uint32_t warp_select_u32(const uint32_t* keys, int n, int k, int* hist) {
+// Lower median (rank (n - 1) / 2, 0-based) of the warp's n keys, lane l
+// holding keys l, l + 32, ... in key[], unused slots 0xffffffff.
+template <int NK>
+__device__ __forceinline__ uint32_t warp_median(const uint32_t (&key)[NK], int n) {
     const int lane = threadIdx.x & 31;
-    uint32_t prefix = 0, mask = 0;
+    uint32_t any = 0, all = 0xffffffffu;  // bits set in some key, in every key
+#pragma unroll
+    for (int j = 0; j < NK; j++)
+        if (lane + 32 * j < n) {
+            any |= key[j];
+            all &= key[j];
+        }
+    any = __reduce_or_sync(0xffffffffu, any);
+    all = __reduce_and_sync(0xffffffffu, all);
+    const uint32_t diff = any ^ all;
+    if (diff == 0) return all;  // all keys equal
+    const int k = (n - 1) / 2;
+    int bit = 31 - __clz(diff);
+    uint32_t lo = bit == 31 ? 0u : all & ~((2u << bit) - 1u);  // the keys' common leading bits
+    int below = 0, upto = n;  // keys < lo, keys < lo + 2^(bit + 1)
 #pragma unroll 1
-    for (int shift = 24; shift >= 0; shift -= 8) {
+    for (; bit >= 0 && upto - below > 1; bit--) {
+        const uint32_t mid = lo | (1u << bit);
+        int c = 0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) hist[lane * 8 + j] = 0;
-        __syncwarp();
-        for (int i0 = 0; i0 < n; i0 += 32) {
-            const int i = i0 + lane;
-            bool act = false;
-            uint32_t d = 0;
-            if (i < n) {
-                const uint32_t key = keys[i];
-                act = (key & mask) == prefix;
-                d = (key >> shift) & 255u;
-            }
-            // aggregate equal digits before the shared-memory atomic
-            const unsigned am = __ballot_sync(0xffffffffu, act);
-            if (act) {
-                const unsigned peers = __match_any_sync(am, d);
-                if (lane == __ffs(peers) - 1) atomicAdd(&hist[d], __popc(peers));
-            }
+        for (int j = 0; j < NK; j++) c += key[j] < mid;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c <= k) {
+            lo = mid;
+            below = c;
+        } else {
+            upto = c;
         }
-        __syncwarp();
-        int loc[8], sum = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            loc[j] = hist[lane * 8 + j];
-            sum += loc[j];
-        }
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int excl = incl - sum;
-        int digit = 0, knew = 0;
-        const bool mine = k >= excl && k < incl;
-        if (mine) {
-            int c = excl;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                if (k >= c && k < c + loc[j]) {
-                    digit = lane * 8 + j;
-                    knew = k - c;
-                }
-                c += loc[j];
-            }
-        }
-        const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
-        digit = __shfl_sync(0xffffffffu, digit, src);
-        k = __shfl_sync(0xffffffffu, knew, src);
-        prefix |= (uint32_t)digit << shift;
-        mask |= 255u << shift;
-        __syncwarp();
     }
-    return prefix;
+    if (bit < 0) return lo;
+    // one key left in [lo, lo + 2^(bit + 1))
+    const uint32_t lead = lo >> bit >> 1;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < NK; j++)
+        if (lane + 32 * j < n && (key[j] >> bit >> 1) == lead) mine = key[j];
+    return __reduce_or_sync(0xffffffffu, mine);
 }
 
+template <int NK>
+__device__ __forceinline__ uint32_t block_median(const float2* __restrict__ spec, int n) {
+    const int lane = threadIdx.x & 31;
+    uint32_t key[NK];
+#pragma unroll
+    for (int j = 0; j < NK; j++) {
+        const int i = lane + 32 * j;
+        key[j] = i < n ? __float_as_uint(power_exact(spec[i])) : 0xffffffffu;
+    }
+    return warp_median<NK>(key, n);
+}
+
+// med[b]: the block's median power (the level's division is left to the
+// scaling kernel).
 __global__ void __launch_bounds__(32 * kWarpsPerCta) k_whiten_medians_warp(const int* __restrict__ bstart,
                                                                            const int* __restrict__ blen,
                                                                            const float2* __restrict__ spec,
-                                                                           double* med, int nblocks, int maxlen) {
-    extern __shared__ uint32_t wsm[];  // per warp: 256 histogram ints, then maxlen keys
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerCta + w;
-    if (b >= nblocks) return;  // whole warps leave; nothing below synchronises the CTA
-    int* hist = reinterpret_cast<int*>(wsm + (size_t)w * (256 + maxlen));
-    uint32_t* keys = wsm + (size_t)w * (256 + maxlen) + 256;
+                                                                           float* __restrict__ med, int nblocks) {
+    const int b = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
+    if (b >= nblocks) return;
     const int s = bstart[b], n = blen[b];
-    for (int i = lane; i < n; i += 32) keys[i] = __float_as_uint(power_exact(spec[s + i]));
-    __syncwarp();
-    const uint32_t k = warp_select_u32(keys, n, (n - 1) / 2, hist);
-    if (lane == 0) med[b] = (double)__uint_as_float(k) / kLn2w;
+    // registers for 128 bins (widths at the default cap 200 reach 87 at 2^21
+    // bins), 256, or the largest block
+    const uint32_t k = n <= 128 ? block_median<4>(spec + s, n)
+                     : n <= 256 ? block_median<8>(spec + s, n)
+                                : block_median<kWarpBlockMax / 32>(spec + s, n);
+    if ((threadIdx.x & 31) == 0) med[b] = __uint_as_float(k);
 }
 
-// Write range r as in k_whiten_scale, one warp per range.
+// Write ranges as in k_whiten_scale, kScaleRanges per CTA: their starts,
+// levels and slopes by one thread each, then a warp per range.
 __global__ void __launch_bounds__(32 * kWarpsPerCta) k_whiten_scale_warp(const int* __restrict__ bstart,
                                                                          const int* __restrict__ blen,
-                                                                         const double* __restrict__ med, int nb,
+                                                                         const float* __restrict__ med, int nb,
                                                                          float2* spec, unsigned numbins,
                                                                          int exact) {
-    const int r = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (r > nb) return;
-    long long lo, hi;
-    float mean_old, dslope;
-    if (r == 0) {
-        lo = 1;
-        hi = bstart[0] + blen[0] / 2;
-        mean_old = (float)med[0];
-        dslope = 0.f;
-        if (lane == 0) spec[0] = make_float2(1.0f, 0.0f);
-    } else if (r < nb) {
-        lo = bstart[r - 1] + blen[r - 1] / 2;
-        hi = bstart[r] + blen[r] / 2;
-        mean_old = (float)med[r - 1];
-        dslope = (float)((med[r] - (double)mean_old) / (0.5 * (blen[r - 1] + blen[r])));
-    } else {
-        lo = bstart[nb - 1] + blen[nb - 1] / 2;
-        hi = numbins;
-        mean_old = (float)med[nb - 1];
-        if (nb >= 2) {
-            const float mo = (float)med[nb - 2];
-            dslope = (float)((med[nb - 1] - (double)mo) / (0.5 * (blen[nb - 2] + blen[nb - 1])));
-        } else {
-            dslope = 1.0f;
+    __shared__ int s_lo[kScaleRanges + 1];
+    __shared__ float s_mean[kScaleRanges], s_slope[kScaleRanges];
+    const int r0 = blockIdx.x * kScaleRanges, nr = min(kScaleRanges, nb + 1 - r0);
+    auto level = [&](int b) { return (double)med[b] / kLn2w; };
+    if (threadIdx.x <= nr) {
+        const int r = r0 + threadIdx.x;
+        s_lo[threadIdx.x] = r == 0 ? 1 : r <= nb ? bstart[r - 1] + blen[r - 1] / 2 : (int)numbins;
+        if (threadIdx.x < nr) {
+            float mean_old, dslope = 0.f;
+            if (r == 0) {
+                mean_old = (float)level(0);
+                spec[0] = make_float2(1.0f, 0.0f);
+            } else if (r < nb) {
+                mean_old = (float)level(r - 1);
+                dslope = (float)((level(r) - (double)mean_old) / (0.5 * (blen[r - 1] + blen[r])));
+            } else {
+                mean_old = (float)level(nb - 1);
+                if (nb >= 2) {
+                    const float mo = (float)level(nb - 2);
+                    dslope = (float)((level(nb - 1) - (double)mo) / (0.5 * (blen[nb - 2] + blen[nb - 1])));
+                } else {
+                    dslope = 1.0f;
+                }
+            }
+            s_mean[threadIdx.x] = mean_old;
+            s_slope[threadIdx.x] = dslope;
         }
     }
-    const float flat = rsqrt_norm(mean_old, exact);
-    for (long long ind = lo + lane; ind < hi; ind += 32) {
-        float norm;
-        if (r == 0) norm = flat;
-        else norm = rsqrt_norm(__fadd_rn(mean_old, __fmul_rn(dslope, (float)(ind - lo))), exact);
-        float2 v = spec[ind];
-        v.x = __fmul_rn(v.x, norm);
-        v.y = __fmul_rn(v.y, norm);
-        spec[ind] = v;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int q = threadIdx.x >> 5; q < nr; q += kWarpsPerCta) {
+        const unsigned lo = (unsigned)s_lo[q], hi = (unsigned)s_lo[q + 1];
+        const float mean_old = s_mean[q], dslope = s_slope[q];
+        if (r0 + q == 0) {
+            const float flat = rsqrt_norm(mean_old, exact);
+            for (unsigned ind = lo + lane; ind < hi; ind += 32) {
+                const float2 v = spec[ind];
+                spec[ind] = make_float2(__fmul_rn(v.x, flat), __fmul_rn(v.y, flat));
+            }
+            continue;
+        }
+        // four bins per lane in flight
+#pragma unroll 1
+        for (unsigned at = lo + lane; at < hi; at += 128) {
+            float2 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (at + 32 * j < hi) v[j] = spec[at + 32 * j];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const unsigned ind = at + 32 * j;
+                if (ind >= hi) break;
+                const float norm = rsqrt_norm(__fadd_rn(mean_old, __fmul_rn(dslope, (float)(ind - lo))), exact);
+                spec[ind] = make_float2(__fmul_rn(v[j].x, norm), __fmul_rn(v[j].y, norm));
+            }
+        }
     }
 }
 
@@ -250,16 +277,12 @@ std::vector<std::pair<int, int>> plan_whiten_blocks(long long numbins, int initb
 int launch_whiten(const int* d_bstart, const int* d_blen, int nblocks, double* d_med, float2* spec,
                   unsigned numbins, int maxlen, cudaStream_t st, int exact) {
     if (maxlen <= kWarpBlockMax) {
-        const size_t smem = sizeof(uint32_t) * (size_t)kWarpsPerCta * (256 + maxlen);
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(k_whiten_medians_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess)
-            return -1;
-        k_whiten_medians_warp<<<(nblocks + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, smem, st>>>(
-            d_bstart, d_blen, spec, d_med, nblocks, maxlen);
+        float* med = reinterpret_cast<float*>(d_med);
+        k_whiten_medians_warp<<<(nblocks + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, st>>>(
+            d_bstart, d_blen, spec, med, nblocks);
         if (cudaGetLastError() != cudaSuccess) return -1;
-        k_whiten_scale_warp<<<(nblocks + kWarpsPerCta) / kWarpsPerCta, 32 * kWarpsPerCta, 0, st>>>(
-            d_bstart, d_blen, d_med, nblocks, spec, numbins, exact);
+        k_whiten_scale_warp<<<nblocks / kScaleRanges + 1, 32 * kWarpsPerCta, 0, st>>>(d_bstart, d_blen, med, nblocks,
+                                                                                    spec, numbins, exact);
         return cudaGetLastError() == cudaSuccess ? 0 : -1;
     }
     size_t smem = sizeof(uint32_t) * (size_t)maxlen;
