@@ -1016,8 +1016,7 @@ int run_search(accel_ctx* c, int ntrials, float2* const* spec, const long long* 
 void free_ctx(accel_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
-    for (auto& kv : c->r2c.plans) cufftDestroy(kv.second);
-    c->r2c.plans.clear();
+    c->r2c.clear();
     for (auto& e : c->pending) {
         cudaEventDestroy(e.a);
         cudaEventDestroy(e.b);

@@ -24,13 +24,21 @@ struct WhitenPlanDev {
 };
 
 // Real-to-complex transforms of any even length from power-of-two C2C
-// plans (rfft.cu).  One thread uses an engine at a time.
+// plans (rfft.cu).  One thread and one stream at a time use an engine (a
+// context waits for its old stream when it is given another).
+struct R2CLength;
 struct R2CEngine {
     std::map<long long, cufftHandle> plans;  // C2C plans by power-of-two length
+    std::map<long long, R2CLength*> lengths; // per half length: phase tables, chirp
+    size_t length_bytes = 0;
+    long long clock = 0;
+    void* work = nullptr;                    // the transforms' working array
+    size_t work_bytes = 0;
     R2CEngine() = default;
     R2CEngine(const R2CEngine&) = delete;
     R2CEngine& operator=(const R2CEngine&) = delete;
     ~R2CEngine();
+    void clear();                            // free everything (the stream is idle)
 };
 // spec[0 .. n/2] = the DFT of the n real samples of x (device, n even), on
 // stream st: 0, -1 on a CUDA or cuFFT error, -2 when scratch memory runs out.
