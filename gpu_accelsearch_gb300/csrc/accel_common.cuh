@@ -144,6 +144,24 @@ ACCEL_HD StepHarm step_harm(long long startr, int uselen, int p, int q, int hw0)
     return g;
 }
 
+// The same for q = 2^lq, with shifts: 64-bit divisions by a variable cost
+// the preparation kernel about 1400 cycles.
+ACCEL_HD long long twice_required_r_shift(long long r2, int p, int lq) {
+    const long long a = 2LL * r2 * p + (1LL << lq);
+    return a >= 0 ? a >> (lq + 1) : -((-a) >> (lq + 1));  // truncates like the division
+}
+ACCEL_HD StepHarm step_harm_shift(long long startr, int uselen, int p, int lq, int hw0) {
+    StepHarm g;
+    const long long a0 = twice_required_r_shift(2 * startr, p, lq);
+    const long long a1 = twice_required_r_shift(2 * startr + uselen - 1, p, lq);
+    g.rlo = a0 >> 1;
+    g.ceilhi = (a1 + 1) >> 1;
+    g.numrs = lq == 0 ? uselen : (int)(2 * (g.ceilhi - g.rlo) + 2);
+    g.lobin = g.rlo - hw0;
+    g.numdata = (int)(g.ceilhi + hw0 - g.lobin + 1);
+    return g;
+}
+
 // addPowers index arithmetic (bpd_gpu_kernels.cu:139-153):
 // rind = (ushort)((subr - rlo_h) * 2), subr = (int)(2 rr f + 0.5) / 2,
 // rr = startr + i/2.
@@ -256,68 +274,95 @@ __device__ __forceinline__ uint32_t block_select_u32(const uint32_t* keys, int n
     return prefix;
 }
 
-// Exact k-th smallest (0-based) of keys the CTA's threads hold themselves:
-// each(f) calls f(key) for every key of the calling thread.  Three radix
-// passes (11, 11 and 10 bits) over a shared histogram of 2048 counters
-// (hist, 16-byte aligned); scratch: 40 ints of shared memory.  All NT
-// threads (a multiple of 32 up to 1024) call it; the result is the same in
-// every thread, and hist may be reused on return.
+// Exact k-th smallest (0-based) of the n keys the CTA's NT threads hold in
+// registers, NK slots each, unused slots 0xffffffff (and no key that large).
+// NT is a multiple of 32 up to 1024, NT NK <= 32736; scratch is shared
+// memory of kSelectScratch 64-bit words.  Every thread gets the result.
 //
-// Positive floats spread over a few dozen of the first pass's bins (8
-// exponent and 3 mantissa bits), so plain shared atomics meet few
-// collisions and one pass leaves about 1/30 of the keys; keys come from
-// registers or global memory.
-constexpr int kSelectBins = 2048;
-template <int NT, class Each>
-__device__ __forceinline__ uint32_t block_rank_select(Each each, int k, uint32_t* hist, int* scratch) {
-    static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t prefix = 0, mask = 0;
+// A search over the key's bits, two a round: each round counts the keys
+// below three thresholds (compares in registers, one redux.sync per warp
+// over the three counts packed in a word, one barrier for the sum over the
+// warps), from the first bit in which the keys differ until one key is left
+// in the interval -- 8 or 9 rounds for thousands of exponentially
+// distributed powers.  A few thousand cycles of latency and no bank
+// conflicts or atomics, against 12000 (64 threads) and 8500 (256 threads)
+// for three passes over a shared histogram.
+constexpr int kSelectScratch = 66;
+template <int NT, int NK>
+__device__ __forceinline__ uint32_t block_select_reg(const uint32_t (&key)[NK], int n, int k,
+                                                     unsigned long long* scratch) {
+    static_assert(NT % 32 == 0 && NT <= 1024 && NK * 32 <= 1023, "whole warps, 10-bit counts");
+    constexpr int W = NT / 32;
+    constexpr uint32_t kNone = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t any = 0, all = kNone;  // bits set in some key, in every key
 #pragma unroll
-    for (int pass = 0; pass < 3; pass++) {
-        constexpr int kBits[3] = {11, 11, 10}, kShift[3] = {21, 10, 0};
-        const int shift = kShift[pass], bins = 1 << kBits[pass];
-        for (int i = tid; i < kSelectBins / 4; i += NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-        each([&](uint32_t key) {
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & (uint32_t)(bins - 1)], 1u);
-        });
-        __syncthreads();
-        // bins [tid PER, tid PER + PER) of every thread, their sums scanned
-        // over the warp and, through scratch, over the CTA
-        constexpr int PER = kSelectBins / NT;
-        uint32_t sum = 0;
-#pragma unroll
-        for (int j = 0; j < PER; j++) sum += hist[tid * PER + j];
-        int incl = (int)sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) scratch[2 + warp] = incl;
-        __syncthreads();
-        int excl = incl - (int)sum;
-        for (int w = 0; w < warp; w++) excl += scratch[2 + w];
-        if (k >= excl && k < excl + (int)sum) {  // exactly one thread
-            int c = excl, d = 0;
-            for (int j = 0; j < PER; j++) {
-                const int h = (int)hist[tid * PER + j];
-                if (k >= c && k < c + h) {
-                    d = tid * PER + j;
-                    scratch[1] = k - c;
-                }
-                c += h;
-            }
-            scratch[0] = d;
-        }
-        __syncthreads();
-        prefix |= (uint32_t)scratch[0] << shift;
-        mask |= (uint32_t)(bins - 1) << shift;
-        k = scratch[1];
-        __syncthreads();
+    for (int j = 0; j < NK; j++) {
+        if (key[j] != kNone) any |= key[j];
+        all &= key[j];
     }
-    return prefix;
+    any = __reduce_or_sync(kNone, any);
+    all = __reduce_and_sync(kNone, all);
+    if constexpr (W > 1) {
+        if (lane == 0) scratch[warp] = any | ((unsigned long long)all << 32);
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            const unsigned long long v = scratch[w];
+            any |= (uint32_t)v;
+            all &= (uint32_t)(v >> 32);
+        }
+    }
+    if ((any ^ all) == 0) return all;  // all keys equal
+    const int top = 31 - __clz(any ^ all);
+    int s = top > 0 ? top - 1 : 0;  // the digit is bits s + 1 and s
+    uint32_t lo = all & ~((4u << s) - 1u);
+    int below = 0, upto = n;  // keys < lo, keys < lo + 4 * 2^s
+#pragma unroll 1
+    for (int round = 1;; round ^= 1) {
+        const uint32_t m1 = lo + (1u << s), m2 = lo + (2u << s), m3 = lo + (3u << s);
+        uint32_t c = 0;
+#pragma unroll
+        for (int j = 0; j < NK; j++) {
+            if (key[j] < m1) c += 1u;
+            if (key[j] < m2) c += 1u << 10;
+            if (key[j] < m3) c += 1u << 20;
+        }
+        c = __reduce_add_sync(kNone, c);
+        int c1 = c & 1023, c2 = (c >> 10) & 1023, c3 = (int)(c >> 20);
+        if constexpr (W > 1) {
+            // rounds alternate between two halves of scratch: one barrier each
+            if (lane == 0)
+                scratch[32 * round + warp] = (unsigned long long)c1 | ((unsigned long long)c2 << 21) |
+                                             ((unsigned long long)c3 << 42);
+            __syncthreads();
+            unsigned long long t = 0;
+#pragma unroll
+            for (int w = 0; w < W; w++) t += scratch[32 * round + w];
+            c1 = (int)(t & 0x1fffff);
+            c2 = (int)((t >> 21) & 0x1fffff);
+            c3 = (int)(t >> 42);
+        }
+        if (c3 <= k) lo = m3, below = c3;
+        else if (c2 <= k) lo = m2, below = c2, upto = c3;
+        else if (c1 <= k) lo = m1, below = c1, upto = c2;
+        else upto = c1;
+        if (s == 0) return lo;
+        if (upto - below == 1) break;
+        s = s >= 2 ? s - 2 : 0;
+    }
+    // one key left in [lo, lo + 2^s)
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < NK; j++)
+        if (key[j] - lo < (1u << s)) mine = key[j];
+    mine = __reduce_or_sync(kNone, mine);
+    if constexpr (W > 1) {
+        if (mine && lane == 0) scratch[64] = mine;
+        __syncthreads();
+        mine = (uint32_t)scratch[64];
+    }
+    return mine;
 }
 #endif  // __CUDACC__
 

@@ -536,45 +536,47 @@ int run_group(accel_ctx* c, const SegDesc* d_segs, int nseg, int seg_base, float
     if (!sum_stream) sum_stream = c->stream;
     float2* dbuf = dh_in ? const_cast<float2*>(dh_in) : c->dbuf;
     float* planes = planes_out ? planes_out : c->planes;
+    // Segment preparation: the power-of-two harmonics in one launch before the
+    // planes; the short-transform ones in another after the power-of-two
+    // classes' planes (the fundamental's first): by then the previous group's
+    // harmonic sum on the other stream has usually left the SMs.
+    auto prep = [&](bool short_ones) -> int {
+        PrepArgs pa{};
+        int mmax = 0;
+        for (int h = 0; h < c->nh; h++) {
+            if ((mixed_radix(c->hp[h].M) > 1) != short_ones) continue;
+            pa.h[pa.nh++] = c->hp[h];
+            mmax = std::max(mmax, c->hp[h].M);
+        }
+        if (!pa.nh) return ACCEL_OK;
+        pa.uselen = c->uselen;
+        pa.exact_rsqrt = c->cfg.exact_rsqrt;
+        pa.segs = d_segs;
+        pa.dbuf = dbuf;
+        pa.dstride = c->dstride;
+        ProfScope ps(c, K_PREP, 1);
+        CKL(launch_prep(short_ones ? pa.h[0].M : mmax, pa, nseg, c->tw, c->stream), "segment preparation");
+        return ACCEL_OK;
+    };
+    int rc = do_prep ? prep(false) : ACCEL_OK;
+    if (rc) return rc;
     bool short_prepped = !do_prep;
     for (int M : c->mvals) {
         if (mixed_radix(M) > 1 && !short_prepped) {
-            // the segments of every short-transform harmonic in one launch,
-            // after the power-of-two classes' planes (the fundamental's
-            // first): by then the previous group's harmonic sum on the other
-            // stream has usually left the SMs
             short_prepped = true;
-            PrepArgs ps{};
-            int k = 0;
-            for (int h = 0; h < c->nh; h++)
-                if (mixed_radix(c->hp[h].M) > 1) ps.h[k++] = c->hp[h];
-            ps.nh = k;
-            ps.uselen = c->uselen;
-            ps.exact_rsqrt = c->cfg.exact_rsqrt;
-            ps.segs = d_segs;
-            ps.dbuf = dbuf;
-            ps.dstride = c->dstride;
-            ProfScope pscope(c, K_PREP, 1);
-            CKL(launch_prep(M, ps, nseg, c->tw, c->stream), "segment preparation");
+            rc = prep(true);
+            if (rc) return rc;
         }
-        PrepArgs pa{};
         PlaneArgs la{};
-        int k = 0, kp = 0, zb = 0;
+        int kp = 0, zb = 0;
         for (int h = 0; h < c->nh; h++) {
             if (c->hp[h].M != M) continue;
-            pa.h[k++] = c->hp[h];
             if (fused && h == 0) continue;
             la.h[kp] = c->hp[h];
             la.h[kp].zbase = zb;
             zb += c->hp[h].numzs;
             kp++;
         }
-        pa.nh = k;
-        pa.uselen = c->uselen;
-        pa.exact_rsqrt = c->cfg.exact_rsqrt;
-        pa.segs = d_segs;
-        pa.dbuf = dbuf;
-        pa.dstride = c->dstride;
         la.nh = kp;
         la.ntpl = zb;
         la.dbuf = dbuf;
@@ -583,10 +585,6 @@ int run_group(accel_ctx* c, const SegDesc* d_segs, int nseg, int seg_base, float
         la.pstride = c->pstride;
         la.use_fp16 = c->cfg.template_fp16;
         la.split = c->plane_split;
-        if (do_prep && mixed_radix(M) == 1) {
-            ProfScope ps(c, K_PREP, 1);
-            CKL(launch_prep(M, pa, nseg, c->tw, c->stream), "segment preparation");
-        }
         if (do_plane && kp > 0) {
             ProfScope ps(c, K_PLANE, 1);
             CKL(launch_plane(M, la, nseg, c->tw, c->stream), "power plane");

@@ -36,6 +36,10 @@ struct GroupSync {
         asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(nthreads) : "memory");
     }
 };
+struct LaneSync {  // transforms of fewer than 32 threads: some lanes of one warp
+    unsigned mask;
+    __device__ __forceinline__ void operator()() const { __syncwarp(mask); }
+};
 template <int M> struct FftShape {
     static constexpr int T = M / 16;
     static constexpr int PADDED = M + M / 16;

@@ -33,10 +33,9 @@ namespace accel {
 constexpr int kPrepShortThreads = 256;
 
 // Dynamic shared memory of the body for R * N2 points: GROUPS padded
-// N2-point buffers and the median keys.
+// N2-point buffers.
 ACCEL_HD constexpr size_t prep_short_smem(int R, int N2) {
-    return sizeof(float2) * (size_t)(((R * (N2 / 16) + 31) / 32 * 32) / (N2 / 16)) * (N2 + N2 / 16) +
-           sizeof(uint32_t) * (size_t)(R * N2);
+    return sizeof(float2) * (size_t)(((R * (N2 / 16) + 31) / 32 * 32) / (N2 / 16)) * (N2 + N2 / 16);
 }
 template <int R, int N2> struct MixedPrepShape {
     static constexpr int T2 = N2 / 16;
@@ -44,7 +43,7 @@ template <int R, int N2> struct MixedPrepShape {
     static constexpr int GROUPS = FFT_THREADS / T2;
     static constexpr int PM2 = FftShape<N2>::PADDED;
     static constexpr size_t SMEM = prep_short_smem(R, N2);
-    static_assert(SMEM == sizeof(float2) * GROUPS * PM2 + sizeof(uint32_t) * R * N2, "layout");
+    static_assert(SMEM == sizeof(float2) * GROUPS * PM2, "layout");
     static_assert(FFT_THREADS <= kPrepShortThreads, "short transform fits the preparation CTA");
 };
 
@@ -52,13 +51,12 @@ template <int R, int N2> struct MixedPrepShape {
 // segment (bpd_search.cu:130-184, :228-240), as k_prep, into decimated order.
 template <int R, int N2>
 __device__ __forceinline__ void prep_short_body(const PrepArgs& a, const HarmPlan& H, const float2* __restrict__ tw,
-                                                unsigned char* smem_raw, int* hist, int* bc, float* s_norm) {
+                                                unsigned char* smem_raw, unsigned long long* scratch, float* s_norm) {
     using S = MixedPrepShape<R, N2>;
     constexpr int T2 = S::T2, PM2 = S::PM2, M = R * N2;
     float2* sm = reinterpret_cast<float2*>(smem_raw);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(sm + S::GROUPS * PM2);
     const SegDesc sd = a.segs[blockIdx.y];
-    const StepHarm g = step_harm(sd.startr, a.uselen, H.p, H.q, H.hw0);
+    const StepHarm g = step_harm_shift(sd.startr, a.uselen, H.p, H.lq, H.hw0);
     const int tid = threadIdx.x;
     const int grp = tid / T2, t = tid - grp * T2;
     const bool real = grp < R;
@@ -72,12 +70,14 @@ __device__ __forceinline__ void prep_short_body(const PrepArgs& a, const HarmPla
         if (real) {
             const long long b = g.lobin + idx;
             if (b >= 0 && b < sd.numbins) v = sd.spec[b];
-            if (idx < numdata) keys[idx] = __float_as_uint(power_exact(v));
         }
         x[0][e] = v;
     }
-    __syncthreads();
-    const uint32_t mk = block_select_u32(keys, numdata, (numdata - 1) / 2, hist, bc);
+    uint32_t key[16];
+#pragma unroll
+    for (int e = 0; e < 16; e++)
+        key[e] = real && R * (t + e * T2) + grp < numdata ? __float_as_uint(power_exact(x[0][e])) : 0xffffffffu;
+    const uint32_t mk = block_select_reg<kPrepShortThreads, 16>(key, numdata, (numdata - 1) / 2, scratch);
     if (tid == 0) *s_norm = rsqrt_norm((float)((double)__uint_as_float(mk) / kLn2), a.exact_rsqrt);
     __syncthreads();
     const float norm = *s_norm;

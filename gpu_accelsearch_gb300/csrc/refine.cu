@@ -60,10 +60,10 @@ __device__ __forceinline__ double2 zadd(double2 a, double2 b) { return make_doub
 // Squared power normalisation of harmonic k of every candidate, as the
 // search applies it to the candidate's step: the squared rsqrt of the
 // segment's median power / ln 2 (bpd_search.cu:144-181).
-constexpr int kNormThreads = 256;
+constexpr int kNormThreads = 512;
+constexpr int kNormKeys = kMaxM / kNormThreads;  // a segment has at most kMaxM bins
 __global__ void __launch_bounds__(kNormThreads) k_refine_norms(const RefineArgs a) {
-    __shared__ __align__(16) uint32_t hist[kSelectBins];
-    __shared__ int scratch[40];
+    __shared__ unsigned long long scratch[kSelectScratch];
     const OptCand& cand = a.in[blockIdx.x];
     const int k = blockIdx.y;
     if (k >= cand.numharm) return;
@@ -71,14 +71,15 @@ __global__ void __launch_bounds__(kNormThreads) k_refine_norms(const RefineArgs 
     const long long nb = a.numbins[cand.trial];
     const int nd = cand.numdata[k];
     const long long lo = cand.lobin[k];
-    auto each = [&](auto f) {
-        for (int i = threadIdx.x; i < nd; i += kNormThreads) {
-            const long long b = lo + i;
-            const float2 v = (b >= 0 && b < nb) ? X[b] : make_float2(0.f, 0.f);
-            f(__float_as_uint(power_exact(v)));
-        }
-    };
-    const uint32_t mk = block_rank_select<kNormThreads>(each, (nd - 1) / 2, hist, scratch);
+    uint32_t key[kNormKeys];
+#pragma unroll
+    for (int j = 0; j < kNormKeys; j++) {
+        const int i = threadIdx.x + j * kNormThreads;
+        const long long b = lo + i;
+        const float2 v = i < nd && b >= 0 && b < nb ? X[b] : make_float2(0.f, 0.f);
+        key[j] = i < nd ? __float_as_uint(power_exact(v)) : 0xffffffffu;
+    }
+    const uint32_t mk = block_select_reg<kNormThreads, kNormKeys>(key, nd, (nd - 1) / 2, scratch);
     if (threadIdx.x == 0) {
         const double nrm = (double)rsqrt_norm((float)((double)__uint_as_float(mk) / kLn2), a.exact_rsqrt);
         a.norm2[(size_t)blockIdx.x * kMaxHarm + k] = nrm * nrm;

@@ -10,6 +10,24 @@ int launch_plane_r5(int N2, const PlaneArgs& a, int nseg, const float2* tw, cuda
 int launch_plane_r6(int N2, const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t st);
 int launch_plane_r7(int N2, const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t st);
 
+template <int M> static int prep_m(const PrepArgs& a, int nseg, const float2* tw, cudaStream_t st) {
+    constexpr size_t smem = PrepShape<M>::SMEM;
+    static std::atomic<unsigned long long> attr{0};
+    int dev = 0;
+    if (attr_pending(attr, &dev)) {
+        if (cudaFuncSetAttribute(k_prep<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_prep<M>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 carveout_for((const void*)k_prep<M>, PrepShape<M>::NT, smem)) != cudaSuccess)
+            return -1;
+        attr_set(attr, dev);
+    }
+    k_prep<M><<<dim3(a.nh, nseg), PrepShape<M>::NT, smem, st>>>(a, tw);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// Segment preparation of the harmonics in a, whose largest half length is M
+// (power-of-two lengths; short lengths have a kernel of their own).
 int launch_prep(int M, const PrepArgs& a, int nseg, const float2* tw, cudaStream_t st) {
     if (mixed_radix(M) > 1) return launch_prep_short(a, nseg, tw, st);  // any short harmonics
     switch (M) {

@@ -29,38 +29,47 @@ namespace accel {
 
 
 // ------------------------------------------------------------------ prep
-template <int M>
-__global__ void __launch_bounds__(M / 16) k_prep(const PrepArgs a, const float2* __restrict__ tw) {
-    constexpr int T = M / 16;
-    constexpr int PM = FftShape<M>::PADDED;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* sm = reinterpret_cast<float2*>(smem_raw);
-    uint32_t* keys = reinterpret_cast<uint32_t*>(sm + PM);
-    __shared__ int hist[256];
-    __shared__ int bc[2];
-    __shared__ float s_norm;
+// One CTA per (harmonic, segment), each running the body of its harmonic's
+// half length M with max(32, M/16) threads (further warps of the CTA leave at
+// once).  A small part of a large search, but the first kernel of every
+// launch group, latency-bound on one chain: gather, median, normalise, FFT.
+// The median was most of it (a digit histogram with match_any per key, over
+// keys in shared memory: 22 us for one segment of 1024 points); with
+// block_select_reg the same launch takes 8 us
+// (cold cache).  One launch for every harmonic replaces one per length.
+template <int M> struct PrepShape {
+    static constexpr int T = M / 16;
+    static constexpr int NT = T < 32 ? 32 : T;  // threads of the median
+    static constexpr size_t SMEM = sizeof(float2) * FftShape<M>::PADDED;
+};
 
-    const HarmPlan& H = a.h[blockIdx.x];
-    const SegDesc sd = a.segs[blockIdx.y];
-    const StepHarm g = step_harm(sd.startr, a.uselen, H.p, H.q, H.hw0);
+template <int M>
+__device__ __forceinline__ void prep_body(const PrepArgs& a, const HarmPlan& H, const float2* __restrict__ tw,
+                                          unsigned char* smem, unsigned long long* scratch, float* s_norm) {
+    constexpr int T = PrepShape<M>::T, NT = PrepShape<M>::NT;
     const int t = threadIdx.x;
+    if (t >= NT) return;  // whole warps: the barriers below count the others
+    const SegDesc sd = a.segs[blockIdx.y];
+    const StepHarm g = step_harm_shift(sd.startr, a.uselen, H.p, H.lq, H.hw0);
     const int numdata = g.numdata < M ? g.numdata : M;  // host checks numdata <= M
+    const bool mine = T >= 32 || t < T;
 
     float2 x[1][16];
+    uint32_t key[16];
 #pragma unroll
     for (int e = 0; e < 16; e++) {
-        const int idx = t + e * T;
-        const long long b = g.lobin + idx;
-        float2 v = make_float2(0.f, 0.f);
-        if (b >= 0 && b < sd.numbins) v = sd.spec[b];
-        x[0][e] = v;
-        if (idx < numdata) keys[idx] = __float_as_uint(power_exact(v));
+        const long long b = g.lobin + t + e * T;
+        x[0][e] = make_float2(0.f, 0.f);
+        if (mine && b >= 0 && b < sd.numbins) x[0][e] = sd.spec[b];
     }
+#pragma unroll
+    for (int e = 0; e < 16; e++)
+        key[e] = mine && t + e * T < numdata ? __float_as_uint(power_exact(x[0][e])) : 0xffffffffu;
+    const uint32_t mk = block_select_reg<NT, 16>(key, numdata, (numdata - 1) / 2, scratch);
+    if (t == 0) *s_norm = rsqrt_norm((float)((double)__uint_as_float(mk) / kLn2), a.exact_rsqrt);
     __syncthreads();
-    const uint32_t mk = block_select_u32(keys, numdata, (numdata - 1) / 2, hist, bc);
-    if (t == 0) s_norm = rsqrt_norm((float)((double)__uint_as_float(mk) / kLn2), a.exact_rsqrt);
-    __syncthreads();
-    const float norm = s_norm;
+    if (!mine) return;
+    const float norm = *s_norm;
 #pragma unroll
     for (int e = 0; e < 16; e++) {
         if (t + e * T < numdata) {
@@ -68,10 +77,34 @@ __global__ void __launch_bounds__(M / 16) k_prep(const PrepArgs a, const float2*
             x[0][e].y = __fmul_rn(x[0][e].y, norm);
         }
     }
-    fft_run<M, -1, 1>(x, sm, tw, t);
+    float2* sm = reinterpret_cast<float2*>(smem);
+    if constexpr (T >= 32) fft_run<M, -1, 1>(x, sm, tw, t);
+    else fft_run<M, -1, 1, LaneSync>(x, sm, tw, t, LaneSync{(1u << T) - 1u});
     float2* out = a.dbuf + (long long)blockIdx.y * a.dstride + H.doff;
 #pragma unroll
     for (int e = 0; e < 16; e++) out[t + e * T] = x[0][e];
+}
+
+// MMAX: the largest half length of the launch.
+template <int MMAX>
+__global__ void __launch_bounds__(PrepShape<MMAX>::NT) k_prep(const PrepArgs a, const float2* __restrict__ tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned long long scratch[kSelectScratch];
+    __shared__ float s_norm;
+    const HarmPlan& H = a.h[blockIdx.x];
+#define ACCEL_PREP_FORM(m)                                                   \
+    if constexpr (MMAX >= m) {                                               \
+        if (H.M == m) prep_body<m>(a, H, tw, smem_raw, scratch, &s_norm);    \
+    }
+    ACCEL_PREP_FORM(8192)
+    ACCEL_PREP_FORM(4096)
+    ACCEL_PREP_FORM(2048)
+    ACCEL_PREP_FORM(1024)
+    ACCEL_PREP_FORM(512)
+    ACCEL_PREP_FORM(256)
+    ACCEL_PREP_FORM(128)
+    ACCEL_PREP_FORM(64)
+#undef ACCEL_PREP_FORM
 }
 
 // ----------------------------------------------------------------- plane
@@ -845,22 +878,6 @@ __global__ void __launch_bounds__(kHsumCols) k_hsum(const HsumArgs a) {
 }
 
 // -------------------------------------------------------------- launchers
-template <int M> static int prep_m(const PrepArgs& a, int nseg, const float2* tw, cudaStream_t st) {
-    size_t smem = sizeof(float2) * FftShape<M>::PADDED + sizeof(uint32_t) * M;
-    static std::atomic<unsigned long long> attr{0};
-    int dev = 0;
-    if (attr_pending(attr, &dev)) {
-        if (cudaFuncSetAttribute(k_prep<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_prep<M>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 carveout_for((const void*)k_prep<M>, M / 16, smem)) != cudaSuccess)
-            return -1;
-        attr_set(attr, dev);
-    }
-    k_prep<M><<<dim3(a.nh, nseg), M / 16, smem, st>>>(a, tw);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
 template <int M, bool F16, bool SPLIT>
 static int plane_m(const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t st) {
     size_t smem = sizeof(float2) * FftShape<M>::PADDED * PlaneShape<SPLIT, M>::BUFFERS;

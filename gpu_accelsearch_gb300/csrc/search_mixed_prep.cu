@@ -14,14 +14,13 @@ constexpr size_t kPrepShortSmem = cmax(prep_short_smem_r<5>(), cmax(prep_short_s
 // One CTA per (short harmonic, segment): the body of the harmonic's length.
 __global__ void __launch_bounds__(kPrepShortThreads) k_prep_short(const PrepArgs a, const float2* __restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int hist[256];
-    __shared__ int bc[2];
+    __shared__ unsigned long long scratch[kSelectScratch];
     __shared__ float s_norm;
     const HarmPlan& H = a.h[blockIdx.x];
     const int R = mixed_radix(H.M), N2 = R > 1 ? H.M / R : 0;
 #define ACCEL_PREP_FORM(r, n)                                                      \
     if (R == r && N2 == n) {                                                       \
-        prep_short_body<r, n>(a, H, tw, smem_raw, hist, bc, &s_norm);              \
+        prep_short_body<r, n>(a, H, tw, smem_raw, scratch, &s_norm);               \
         return;                                                                    \
     }
     ACCEL_PREP_FORM(5, 64) ACCEL_PREP_FORM(5, 128) ACCEL_PREP_FORM(5, 256) ACCEL_PREP_FORM(5, 512)
