@@ -394,28 +394,32 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// Tensor maps of the tiled sum's boxes for both plane buffers: harmonic h
-// as a 3-D tensor (prow_h columns, numzs_h rows, chunk segments; strides
-// prow_h and pstride floats) starting at its plane offset.  A plan, height
-// or buffer whose maps cannot be made takes the per-row bulk copies.
-void encode_hsum_maps(accel_ctx* c) {
+// Tensor maps of the tiled sum's boxes of height index k over the planes of
+// nseg segments at `planes` (16-byte aligned): harmonic h as a 3-D tensor
+// (prow_h columns, numzs_h rows, nseg segments; strides prow_h and pstride
+// floats) starting at its plane offset.  False where they cannot be made:
+// the sum then takes the per-row bulk copies.
+bool encode_maps(const accel_ctx* c, float* planes, int nseg, int k, HsumMaps* out) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    bool ok = enc && planes && c->tbox_ok[k];
+    for (int h = 0; h < c->nh && ok; h++) {
+        const HarmPlan& H = c->hp[h];
+        const cuuint64_t dim[3] = {(cuuint64_t)H.prow, (cuuint64_t)H.numzs, (cuuint64_t)nseg};
+        const cuuint64_t stride[2] = {(cuuint64_t)H.prow * 4, (cuuint64_t)c->pstride * 4};
+        const cuuint32_t box[3] = {(cuuint32_t)(4 * c->tbox_w4[k][h]), (cuuint32_t)c->tbox_h[k][h], 1};
+        const cuuint32_t estr[3] = {1, 1, 1};
+        ok = enc(&out->m[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, planes + H.poff, dim, stride, box, estr,
+                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    return ok;
+}
+
+// The maps of the context's own two plane buffers, for every tile height.
+void encode_hsum_maps(accel_ctx* c) {
     float* bufs[2] = {c->planes, c->planes2};
     for (int b = 0; b < 2; b++)
-        for (int k = 0; k < 3; k++) {
-            bool ok = enc && bufs[b] && c->tbox_ok[k];
-            for (int h = 0; h < c->nh && ok; h++) {
-                const HarmPlan& H = c->hp[h];
-                const cuuint64_t dim[3] = {(cuuint64_t)H.prow, (cuuint64_t)H.numzs, (cuuint64_t)c->chunk};
-                const cuuint64_t stride[2] = {(cuuint64_t)H.prow * 4, (cuuint64_t)c->pstride * 4};
-                const cuuint32_t box[3] = {(cuuint32_t)(4 * c->tbox_w4[k][h]), (cuuint32_t)c->tbox_h[k][h], 1};
-                const cuuint32_t estr[3] = {1, 1, 1};
-                ok = enc(&c->tmaps[b][k].m[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, bufs[b] + H.poff, dim, stride,
-                         box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-            }
-            c->tmaps_ok[b][k] = ok;
-        }
+        for (int k = 0; k < 3; k++) c->tmaps_ok[b][k] = encode_maps(c, bufs[b], c->chunk, k, &c->tmaps[b][k]);
 }
 
 int alloc_work(accel_ctx* c) {
@@ -644,19 +648,21 @@ int run_group(accel_ctx* c, const SegDesc* d_segs, int nseg, int seg_base, float
         ProfScope ps(c, K_HSUM, 1, sum_stream);
         c->stats.segments += nseg;
         c->stats.cells += (long long)nseg * c->uselen * c->numzs0;
+        // the tuned tile height where its tiles fit, else 16 rows, else 8
+        int k = c->tile_rows == 8 ? 0 : c->tile_rows == 32 ? 2 : 1;
+        if (!c->tile_ok_h[k]) k = 1;
+        if (!c->tile_ok_h[k]) k = 0;
         if (c->tile_ok && c->hsum_tiled && c->hsum_pipe && 4LL * ((c->tile_floats + 31) & ~31) * kPipeBuffers <= kPipeSmemMax)
             CKL(launch_hsum_pipe(ha, nseg, sum_stream), "harmonic sum (tiled, pipelined)");
-        else if (c->tile_ok && c->hsum_tiled) {
-            // the tuned tile height where its tiles fit, else 16 rows
-            int k = c->tile_rows == 8 ? 0 : c->tile_rows == 32 ? 2 : 1;
-            if (!c->tile_ok_h[k]) k = 1;
+        else if (c->tile_ok_h[k] && c->hsum_tiled) {
             ha.tile_floats = c->tile_floats_h[k];
-            // one box copy per harmonic where the planes are one of the
-            // context's two buffers and their maps exist
+            // one box copy per harmonic: maps of the context's buffers, or
+            // made here for planes of the caller's
             const int b = planes == c->planes ? 0 : planes == c->planes2 ? 1 : -1;
             const HsumMaps* maps = nullptr;
-            if (c->hsum_tensor && b >= 0 && c->tmaps_ok[b][k]) {
-                maps = &c->tmaps[b][k];
+            HsumMaps own;
+            if (c->hsum_tensor && (b >= 0 ? c->tmaps_ok[b][k] : encode_maps(c, planes, nseg, k, &own))) {
+                maps = b >= 0 ? &c->tmaps[b][k] : &own;
                 ha.use_tmap = 1;
                 for (int h = 0; h < c->nh; h++) {
                     ha.box_w4[h] = c->tbox_w4[k][h];

@@ -532,10 +532,12 @@ __device__ __forceinline__ bool hsum_tile_body(const HsumArgs& a, int seg, int z
 
     // 4. sums in the reference's harmonic order, RB rows at a time (their
     //    row offsets in one vector load per harmonic); one warp vote per
-    //    row over all stage tests, the per-stage appends only when some
-    //    lane hit
+    //    row over all stage tests, its hits counted only when some lane hit
     constexpr int RB = (NH <= 8 && !STAGE_OUT) ? 4 : 2;  // rows per batch (registers)
     const char* tb = reinterpret_cast<const char*>(tsm);
+    unsigned hit_rows = 0;  // rows of the tile with a hit in this warp
+    int hits = 0;           // their candidates, all stages
+    static_assert(TZ <= 32, "one bit per row");
 #pragma unroll 1
     for (int zq = 0; zq < nz; zq += RB) {
         int ro[NH][RB];
@@ -575,13 +577,45 @@ __device__ __forceinline__ bool hsum_tile_body(const HsumArgs& a, int seg, int z
                 }
             }
             if (__any_sync(0xffffffffu, live && any)) {
+                hit_rows |= 1u << zr;
 #pragma unroll
-                for (int h = 0; h < NH; h++) {
-                    const int st = stage_after(h);
-                    if (st >= 0)
-                        append_candidates(live && sst[st] > cut[st], a.seg_base + seg, i, z, h + 1, sst[st],
-                                          a.cands, a.ncand, a.cap);
+                for (int st = 0; st <= stage_after(NH - 1); st++)
+                    hits += __popc(__ballot_sync(0xffffffffu, live && sst[st] > cut[st]));
+            }
+        }
+    }
+    // 5. one reservation per warp for all of its candidates, then the rows
+    //    that have some once more (the same sums, from shared memory): a
+    //    reservation per row and stage left a tile on a signal waiting on up
+    //    to 16 x 4 atomics in turn, 18 us for a one-segment launch against
+    //    10 us with this (cold cache)
+    if (hits == 0) return true;  // warp-uniform; nothing below synchronises the CTA
+    unsigned long long slot = 0;
+    if ((tid & 31) == 0) slot = atomicAdd(a.ncand, (unsigned long long)hits);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll 1
+    for (; hit_rows; hit_rows &= hit_rows - 1) {
+        const int zr = __ffs(hit_rows) - 1;
+        float s = 0.f;
+#pragma unroll
+        for (int h = 0; h < NH; h++) {
+            const float v = *reinterpret_cast<const float*>(tb + S.row[h][zr] + colb[h]);
+            s = (h == 0) ? v : s + v;
+            const int st = stage_after(h);
+            if (st >= 0) {
+                const bool hit = valid && s > cut[st];
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                const unsigned long long at = slot + __popc(m & ((1u << (tid & 31)) - 1u));
+                if (hit && (long long)at < a.cap) {
+                    RawCand c;
+                    c.seg = a.seg_base + seg;
+                    c.ridx = i;
+                    c.zidx = (int16_t)(z0 + zr);
+                    c.numharm = (int16_t)(h + 1);
+                    c.power = s;
+                    a.cands[at] = c;
                 }
+                slot += __popc(m);
             }
         }
     }
