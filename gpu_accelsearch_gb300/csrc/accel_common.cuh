@@ -26,10 +26,12 @@ constexpr double kLn2 = 0.693147180559945309417232121458;  // median -> mean of 
 constexpr int kFintBins = 16;       // NUMFINTBINS (bpd_common.h:45)
 constexpr int kTwN = 8192;          // twiddle table length (max FFT points)
 // Behind the kTwN-entry table: for every later-pass length NR of the
-// shared-memory FFT, the base twiddles W^k, W^2k, W^4k, W^8k of pass index k
-// (W = exp(2 pi i / NR)) side by side, four float2 per k, so that a thread
-// fetches its pass's base twiddles with two 16-byte loads from consecutive
-// memory instead of four scattered ones.  Sections: NR = 64, 128, 256 (16
+// shared-memory FFT, the base twiddles of pass index k (W = exp(2 pi i / NR))
+// in two planes, (W^k, W^2k) of every k and then (W^4k, W^8k) of every k, so
+// that the threads of a warp fetch theirs by 16-byte loads of consecutive
+// memory (with the four side by side, 32 bytes apart, each such load took 16
+// wavefronts of the L1 data pipe instead of 4, and it is this pipe that the
+// plane kernels fill: 92 % at 2048 points).  Sections: NR = 64, 128, 256 (16
 // entries each), 512, 1024, 2048, 4096 (256 entries each).
 ACCEL_HD constexpr int tw_pack_entries(int NR) { return NR <= 256 ? 16 : 256; }
 ACCEL_HD constexpr int tw_pack_off(int NR) {  // in float2, from the start of the packed part

@@ -275,7 +275,9 @@ __global__ void k_twiddles(float2* tw) {
         int NR = 64;
         for (int j = 0; j < 7; j++)
             if (p >= tw_pack_off(nrs[j])) NR = nrs[j];
-        const int q = p - tw_pack_off(NR), k = q >> 2, slot = q & 3;
+        // two planes of (W^k, W^2k) and (W^4k, W^8k)
+        const int q = p - tw_pack_off(NR), plane = q / (2 * tw_pack_entries(NR));
+        const int k = (q >> 1) % tw_pack_entries(NR), slot = 2 * plane + (q & 1);
         m = ((1 << slot) * k * (kTwN / NR)) & (kTwN - 1);
     }
     double s, c;

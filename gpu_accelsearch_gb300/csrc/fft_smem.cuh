@@ -45,6 +45,40 @@ template <int M> struct FftShape {
     static constexpr int PADDED = M + M / 16;
 };
 
+// Sums and scaled sums of complex numbers, PK: both components in one packed
+// instruction (add/sub/fma.rn.f32x2, the same roundings as two).  A packed
+// instruction holds the FP32 pipe as long as two, so what it saves is issue
+// slots: 54 -> 45 instructions per point, which moves the plane kernels 2 to 3
+// % (their L1 data pipe is the busier unit).  The 8192-point transform (one
+// CTA of 16 warps per SM) is 3 % slower packed and keeps the scalar forms.
+template <bool PK> __device__ __forceinline__ float2 padd(float2 a, float2 b) {
+    if constexpr (!PK) return cadd(a, b);
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n"
+        " mov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <bool PK> __device__ __forceinline__ float2 psub(float2 a, float2 b) {
+    if constexpr (!PK) return csub(a, b);
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.f32x2 x, x, y;\n"
+        " mov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <bool PK> __device__ __forceinline__ float2 pfma(float s, float2 a, float2 b) {  // s a + b
+    if constexpr (!PK) return make_float2(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y));
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %2};\n mov.b64 y, {%3, %4};\n mov.b64 z, {%5, %6};\n"
+        " fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(s), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
 // x * (DIR * i)
 template <int DIR> __device__ __forceinline__ float2 mul_i(float2 a) {
     return DIR > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
@@ -56,11 +90,11 @@ template <int DIR> __device__ __forceinline__ void dft2(float2* v) {
     v[1] = csub(a, b);
 }
 
-template <int DIR> __device__ __forceinline__ void dft4(float2* v) {
-    float2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-    float2 s13 = cadd(v[1], v[3]), d13 = mul_i<DIR>(csub(v[1], v[3]));
-    v[0] = cadd(s02, s13);
-    v[2] = csub(s02, s13);
+template <int DIR, bool PK> __device__ __forceinline__ void dft4(float2* v) {
+    float2 s02 = padd<PK>(v[0], v[2]), d02 = psub<PK>(v[0], v[2]);
+    float2 s13 = padd<PK>(v[1], v[3]), d13 = mul_i<DIR>(psub<PK>(v[1], v[3]));
+    v[0] = padd<PK>(s02, s13);
+    v[2] = psub<PK>(s02, s13);
     v[1] = cadd(d02, d13);
     v[3] = csub(d02, d13);
 }
@@ -81,22 +115,21 @@ __device__ __forceinline__ float2 cfma(float s, float2 a, float2 b) {  // s a + 
     return make_float2(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y));
 }
 
-
 // 8 points as 2 x 4; the twiddles W8^1 = s (1 + i'), W8^3 = s (-1 + i')
 // (i' = DIR i, s = 1/sqrt2) applied by the fused multiply-adds of the last
 // layer: 52 floating-point instructions instead of 56.
-template <int DIR> __device__ __forceinline__ void dft8(float2* v) {
+template <int DIR, bool PK> __device__ __forceinline__ void dft8(float2* v) {
     const float S = 0.70710678118654752440f;
     float2 e[4] = {v[0], v[2], v[4], v[6]};
     float2 o[4] = {v[1], v[3], v[5], v[7]};
-    dft4<DIR>(e);
-    dft4<DIR>(o);
+    dft4<DIR, PK>(e);
+    dft4<DIR, PK>(o);
     const float2 p1 = cadd(o[1], mul_i<DIR>(o[1])), p3 = csub(mul_i<DIR>(o[3]), o[3]);
     const float2 o2 = mul_i<DIR>(o[2]);
-    v[0] = cadd(e[0], o[0]), v[4] = csub(e[0], o[0]);
-    v[1] = cfma(S, p1, e[1]), v[5] = cfma(-S, p1, e[1]);
+    v[0] = padd<PK>(e[0], o[0]), v[4] = psub<PK>(e[0], o[0]);
+    v[1] = pfma<PK>(S, p1, e[1]), v[5] = pfma<PK>(-S, p1, e[1]);
     v[2] = cadd(e[2], o2), v[6] = csub(e[2], o2);
-    v[3] = cfma(S, p3, e[3]), v[7] = cfma(-S, p3, e[3]);
+    v[3] = pfma<PK>(S, p3, e[3]), v[7] = pfma<PK>(-S, p3, e[3]);
 }
 
 // 16 points as 4 x 4: x[4 n1 + n2] -> X[k1 + 4 k2].  DFT4 over n1 for each
@@ -108,54 +141,54 @@ template <int DIR> __device__ __forceinline__ void dft8(float2* v) {
 // multiply-adds of the second DFT4 layer, whose two inputs of a pair carry
 // the same scale: 144 floating-point instructions per 16 points instead of
 // 160 with the twiddles multiplied out.
-template <int DIR> __device__ __forceinline__ void dft16(float2* v) {
+template <int DIR, bool PK> __device__ __forceinline__ void dft16(float2* v) {
     const float C = 0.92387953251128675613f, S = 0.70710678118654752440f, TN = 0.41421356237309504880f;
     float2 y[4][4];  // y[n2][k1]
 #pragma unroll
     for (int n2 = 0; n2 < 4; n2++) {
         float2 u[4] = {v[n2], v[n2 + 4], v[n2 + 8], v[n2 + 12]};
-        dft4<DIR>(u);
+        dft4<DIR, PK>(u);
 #pragma unroll
         for (int k1 = 0; k1 < 4; k1++) y[n2][k1] = u[k1];
     }
     {  // k1 = 0: no twiddles
         float2 u[4] = {y[0][0], y[1][0], y[2][0], y[3][0]};
-        dft4<DIR>(u);
+        dft4<DIR, PK>(u);
         v[0] = u[0], v[4] = u[1], v[8] = u[2], v[12] = u[3];
     }
     {  // k1 = 1: W^1 = c (1 + t i'), W^2 = s (1 + i'), W^3 = c (t + i')
         const float2 p2 = cadd(y[2][1], mul_i<DIR>(y[2][1]));
-        const float2 s02 = cfma(S, p2, y[0][1]), d02 = cfma(-S, p2, y[0][1]);
+        const float2 s02 = pfma<PK>(S, p2, y[0][1]), d02 = pfma<PK>(-S, p2, y[0][1]);
         const float2 i1 = mul_i<DIR>(y[1][1]), i3 = mul_i<DIR>(y[3][1]);
         const float2 a1 = cfma(TN, i1, y[1][1]), a3 = cfma(TN, y[3][1], i3);
-        const float2 s13 = cadd(a1, a3), d13 = mul_i<DIR>(csub(a1, a3));
-        v[1] = cfma(C, s13, s02), v[9] = cfma(-C, s13, s02);
+        const float2 s13 = padd<PK>(a1, a3), d13 = mul_i<DIR>(psub<PK>(a1, a3));
+        v[1] = pfma<PK>(C, s13, s02), v[9] = pfma<PK>(-C, s13, s02);
         v[5] = cfma(C, d13, d02), v[13] = cfma(-C, d13, d02);
     }
     {  // k1 = 2: W^2 = s (1 + i'), W^4 = i', W^6 = s (-1 + i')
         const float2 i2 = mul_i<DIR>(y[2][2]);
         const float2 s02 = cadd(y[0][2], i2), d02 = csub(y[0][2], i2);
-        const float2 a = csub(y[1][2], y[3][2]), ib = mul_i<DIR>(cadd(y[1][2], y[3][2]));
+        const float2 a = psub<PK>(y[1][2], y[3][2]), ib = mul_i<DIR>(padd<PK>(y[1][2], y[3][2]));
         const float2 s13 = cadd(a, ib), d13 = csub(ib, a);
-        v[2] = cfma(S, s13, s02), v[10] = cfma(-S, s13, s02);
-        v[6] = cfma(S, d13, d02), v[14] = cfma(-S, d13, d02);
+        v[2] = pfma<PK>(S, s13, s02), v[10] = pfma<PK>(-S, s13, s02);
+        v[6] = pfma<PK>(S, d13, d02), v[14] = pfma<PK>(-S, d13, d02);
     }
     {  // k1 = 3: W^3 = c (t + i'), W^6 = s (-1 + i'), W^9 = -c (1 + t i')
         const float2 p2 = csub(mul_i<DIR>(y[2][3]), y[2][3]);
-        const float2 s02 = cfma(S, p2, y[0][3]), d02 = cfma(-S, p2, y[0][3]);
+        const float2 s02 = pfma<PK>(S, p2, y[0][3]), d02 = pfma<PK>(-S, p2, y[0][3]);
         const float2 i1 = mul_i<DIR>(y[1][3]), i3 = mul_i<DIR>(y[3][3]);
         const float2 a1 = cfma(TN, y[1][3], i1), a3 = cfma(TN, i3, y[3][3]);
-        const float2 s13 = csub(a1, a3), d13 = mul_i<DIR>(cadd(a1, a3));
-        v[3] = cfma(C, s13, s02), v[11] = cfma(-C, s13, s02);
+        const float2 s13 = psub<PK>(a1, a3), d13 = mul_i<DIR>(padd<PK>(a1, a3));
+        v[3] = pfma<PK>(C, s13, s02), v[11] = pfma<PK>(-C, s13, s02);
         v[7] = cfma(C, d13, d02), v[15] = cfma(-C, d13, d02);
     }
 }
 
-template <int R, int DIR> __device__ __forceinline__ void dft(float2* v) {
+template <int R, int DIR, bool PK = true> __device__ __forceinline__ void dft(float2* v) {
     if constexpr (R == 2) dft2<DIR>(v);
-    else if constexpr (R == 4) dft4<DIR>(v);
-    else if constexpr (R == 8) dft8<DIR>(v);
-    else dft16<DIR>(v);
+    else if constexpr (R == 4) dft4<DIR, PK>(v);
+    else if constexpr (R == 8) dft8<DIR, PK>(v);
+    else dft16<DIR, PK>(v);
 }
 
 template <int DIR> __device__ __forceinline__ float2 twid(const float2* __restrict__ tw, int idx) {
@@ -164,8 +197,8 @@ template <int DIR> __device__ __forceinline__ float2 twid(const float2* __restri
 }
 
 // The base twiddles W^k, W^2k, W^4k, W^8k (W = exp(DIR 2 pi i / NR)) of
-// pass index k: from the packed section of NR (two 16-byte loads of
-// consecutive memory) or, for NR = kTwN, from the table itself.
+// pass index k: from the two planes of NR's packed section (16-byte loads
+// of consecutive memory) or, for NR = kTwN, from the table itself.
 struct Tw16 {
     float2 w1, w2, w4, w8;
 };
@@ -179,8 +212,8 @@ __device__ __forceinline__ Tw16 load_tw16(const float2* __restrict__ tw, int k, 
         r.w8 = twid<DIR>(tw, (8 * k) & (kTwN - 1));
         return r;
     }
-    const float4* p = reinterpret_cast<const float4*>(tw + kTwN + tw_pack_off(NR)) + 2 * k;
-    const float4 a = __ldg(p), b = __ldg(p + 1);
+    const float4* p = reinterpret_cast<const float4*>(tw + kTwN + tw_pack_off(NR)) + k;
+    const float4 a = __ldg(p), b = __ldg(p + tw_pack_entries(NR));
     const float sg = DIR > 0 ? 1.f : -1.f;
     r.w1 = make_float2(a.x, sg * a.y);
     r.w2 = make_float2(a.z, sg * a.w);
@@ -308,7 +341,7 @@ __device__ __forceinline__ void fft_pass(float2 (&a)[NB][16], float2* sm,
         const int jp = fft_pad((b / NS) * (NS * R) + k);
 #pragma unroll
         for (int nb = 0; nb < NB; nb++) {
-            dft<R, DIR>(v[nb]);
+            dft<R, DIR, (M < 8192)>(v[nb]);
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 if constexpr (LAST) a[nb][q + r * Q] = v[nb][r];

@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLI
 #pragma unroll
         for (int e = 0; e < 16; e++) {
             const int i2 = t + e * T - H.hw0;  // one unsigned compare for 0 <= i2 < half_w
-            if ((unsigned)i2 < (unsigned)half_w) *reinterpret_cast<float2*>(row + 2 * i2) = p[e];
+            // (streaming: the row is next read by the harmonic sum)
+            if ((unsigned)i2 < (unsigned)half_w) __stcs(reinterpret_cast<float2*>(row + 2 * i2), p[e]);
         }
     } else {
         // even transform, then odd, each stored as it completes (a loop, not
