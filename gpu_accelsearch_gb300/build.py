@@ -30,7 +30,7 @@ SOURCES = ["api.cu", "bank.cu", "search.cu", "search_plane_lo.cu", "search_plane
            "search_mixed6.cu", "search_mixed7.cu", "search_mixed_prep.cu", "refine.cu"]
 EXTRA = {"bank.cu": ["-fmad=false"], "compat.cu": ["-Xcompiler", "-ffp-contract=off"],
          "dedisperse.cu": ["-Xcompiler", "-ffp-contract=off"]}
-HEADERS = ["accel_common.cuh", "accel_internal.h", "context.h", "fft_smem.cuh", "search_kernels.cuh",
+HEADERS = ["accel_common.cuh", "accel_internal.h", "async_copy.cuh", "context.h", "fft_smem.cuh", "search_kernels.cuh",
            "step_kernel.cuh", "fft_mixed.cuh", "mixed_kernels.cuh"]
 
 

@@ -23,10 +23,12 @@
 // delays lie close enough together for shared-memory windows.
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "../../include/accelsearch.h"
 #include "accel_internal.h"
+#include "async_copy.cuh"
 
 namespace accel {
 
@@ -90,100 +92,220 @@ __global__ void __launch_bounds__(kDdThreads) k_dedisperse(const float* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Windowed form (the default where its windows fit): a CTA owns kDwD DM
-// trials x kDdThreads*kDdPer output samples.  For each chunk of kDwC
-// channels it copies, per channel, the window of input samples its trials
-// read -- [t0 + wmin_c, t0 + T + wmax_c) with wmin_c / wmax_c the smallest /
-// largest delay of the tile's trials in channel c -- into shared memory by
-// asynchronous copies (cp.async, 4 bytes each, zero-filled past the end of
-// the series), double-buffered so that chunk k+1 lands while chunk k is
-// summed; each sample copied once serves all kDwD trials.  The sums are
-// the same rounded float adds in the same channel order as k_dedisperse.
-constexpr int kDwD = 16;  // DM trials per CTA
-constexpr int kDwC = 8;   // channels per chunk
+// Windowed form (the default where its windows fit): a CTA owns D DM trials x
+// kDdThreads * P output samples.  Per channel, the window of input samples
+// its trials read -- from the tile's smallest to its largest delay -- is
+// brought into shared memory by one bulk asynchronous copy, kDwC channels a
+// stage in a ring of kDwS stages (full: an mbarrier per stage; empty: one CTA
+// barrier per stage), and every copied sample serves all D trials.  The sums
+// are the same rounded float adds in the same channel order as k_dedisperse.
+//
+// A bulk copy starts on a 16-byte boundary: the host rounds each window's
+// start down and adds the remainder (0..3 samples, the same for every time
+// tile) to the trials' offsets.  A window whose rounded range would leave
+// the filterbank (the last channel's end, a first row at an odd address) is
+// copied sample by sample instead.
+//
+// Every addition reads its sample from shared memory, so the kernel is bound
+// by the shared-memory pipe: at one 128-byte wavefront per clock 3.4e10
+// additions (1024 channels, 128 trials, 2^18 samples) take 3.4 ms.  With the
+// windows copied by 4-byte cp.async and 32-bit offsets read one at a time,
+// those took a fifth of the pipe and a CTA-wide wait every 8 channels: 6.1 ms;
+// this form 4.4 ms (77 % of that bound).  Two stages of 8 channels measured the
+// same here and 1.63 against 1.34 ms at 300 channels and a DM step of 3; three
+// CTAs per SM (85 registers) 4.7 ms.
+constexpr int kDwC = 4;   // channels per stage
+constexpr int kDwS = 3;   // stages
+constexpr size_t kDwSmemMax = 110 * 1024;  // two CTAs per SM
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0)
-                 : "memory");
+constexpr int kDwT = kDdThreads * kDdPer;  // output samples per CTA
+
+__device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n"
+        " mov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
 }
 
-// rel [ndtile][nchan][kDwD]: delay - wmin of the tile's trials (0 for padding
-// trials); wmin [ndtile][nchan]; every window fits wlen floats.
+template <int D>
 __global__ void __launch_bounds__(kDdThreads, 2)
-    k_dedisperse_win(const float* __restrict__ in, int nchan, long long nsamp, const int* __restrict__ rel,
-                     const int* __restrict__ wmin, int ndm, int ndtile, int wlen, float* __restrict__ out,
+    k_dedisperse_win(const float* __restrict__ in, int nchan, long long total, const long long* __restrict__ start,
+                     const unsigned short* __restrict__ offs, int ndm, int ndtile, int wlen, float* __restrict__ out,
                      long long nout) {
-    extern __shared__ __align__(16) float dsm[];  // [2][kDwC][wlen] windows, then [2][kDwC][kDwD] delays
-    int* sdel = reinterpret_cast<int*>(dsm + 2 * kDwC * wlen);
+    constexpr int P = kDdPer;
+    extern __shared__ __align__(128) float dsm[];  // [kDwS][kDwC][wlen] windows, then [kDwS][kDwC][D] offsets
+    unsigned short* soff = reinterpret_cast<unsigned short*>(dsm + kDwS * kDwC * wlen);
+    __shared__ __align__(8) unsigned long long full[kDwS];
     const long long bid = blockIdx.x;
     const int tile = (int)(bid % ndtile);
-    const int d0 = tile * kDwD;
-    const long long t0 = (bid / ndtile) * (long long)(kDdThreads * kDdPer);
+    const int d0 = tile * D;
+    const long long t0 = (bid / ndtile) * (long long)kDwT;
     const int tid = threadIdx.x;
-    const int nd = min(kDwD, ndm - d0);
-    const int nchunk = (nchan + kDwC - 1) / kDwC;
-    auto stage = [&](int k, int buf) {
-        const int c0 = k * kDwC;
-        for (int i = tid; i < kDwC * kDwD; i += kDdThreads) {
-            const int c = c0 + i / kDwD;
-            sdel[(buf * kDwC + i / kDwD) * kDwD + i % kDwD] =
-                c < nchan ? rel[((long long)tile * nchan + c) * kDwD + i % kDwD] : 0;
-        }
-        for (int cc = 0; cc < kDwC; cc++) {
-            const int c = c0 + cc;
-            if (c >= nchan) break;
-            const long long base = t0 + wmin[(long long)tile * nchan + c];
-            const float* row = in + (long long)c * nsamp;
-            float* dst = dsm + (buf * kDwC + cc) * wlen;
-            for (int x = tid; x < wlen; x += kDdThreads) {
-                const long long idx = base + x;
-                const bool ok = idx < nsamp;
-                cp_async4(dst + x, row + (ok ? idx : 0), ok);
+    const int nstage = (nchan + kDwC - 1) / kDwC;
+    if (tid == 0)
+        for (int s = 0; s < kDwS; s++) mbar_init(&full[s], 1);
+    __syncthreads();
+    // fill the ring slot of stage k (every thread calls it)
+    auto fill = [&](int k) {
+        const int slot = k % kDwS, c0 = k * kDwC, nc = min(kDwC, nchan - c0);
+        const long long* __restrict__ st = start + (long long)tile * nchan + c0;
+        unsigned bytes = 0;
+        for (int cc = 0; cc < nc; cc++) {
+            const long long at = st[cc] + t0;
+            if (at >= 0 && at + wlen <= total) {
+                bytes += 4u * (unsigned)wlen;
+            } else {  // uniform: this window leaves the filterbank
+                float* dst = dsm + (slot * kDwC + cc) * wlen;
+                for (int x = tid; x < wlen; x += kDdThreads)
+                    dst[x] = at + x >= 0 && at + x < total ? in[at + x] : 0.f;
             }
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        if (tid == 0) {
+            // samples copied one by one for this slot's earlier stages come
+            // before the bulk writes
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            constexpr unsigned ob = 2u * D * kDwC;
+            mbar_arrive_expect_tx(&full[slot], bytes + ob);
+            bulk_copy_g2s(soff + slot * kDwC * D, offs + ((long long)tile * nstage + k) * kDwC * D, ob, &full[slot]);
+            for (int cc = 0; cc < nc; cc++) {
+                const long long at = st[cc] + t0;
+                if (at >= 0 && at + wlen <= total)
+                    bulk_copy_g2s(dsm + (slot * kDwC + cc) * wlen, in + at, 4u * (unsigned)wlen, &full[slot]);
+            }
+        }
     };
-    float acc[kDwD][kDdPer];
+    float2 acc[D][P / 2];
 #pragma unroll
-    for (int j = 0; j < kDwD; j++)
+    for (int j = 0; j < D; j++)
 #pragma unroll
-        for (int q = 0; q < kDdPer; q++) acc[j][q] = 0.f;
-    stage(0, 0);
+        for (int q = 0; q < P / 2; q++) acc[j][q] = make_float2(0.f, 0.f);
+    for (int k = 0; k < kDwS - 1 && k < nstage; k++) fill(k);
+    bool landed = true;
 #pragma unroll 1
-    for (int k = 0; k < nchunk; k++) {
-        const int buf = k & 1;
-        if (k + 1 < nchunk) {
-            stage(k + 1, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // chunk k has landed
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
+    for (int k = 0; k < nstage; k++) {
+        const int slot = k % kDwS;
+        // everyone is done with stage k - 1 (its slot is refilled now) and
+        // sees the samples copied one by one for stage k
         __syncthreads();
-        const int ncc = min(kDwC, nchan - k * kDwC);
-#pragma unroll 1
-        for (int cc = 0; cc < ncc; cc++) {
-            const float* w = dsm + (buf * kDwC + cc) * wlen + tid;
-            const int* dl = sdel + (buf * kDwC + cc) * kDwD;
+        if (k + kDwS - 1 < nstage) fill(k + kDwS - 1);
+        if (!mbar_wait_bounded(&full[slot], (unsigned)(k / kDwS) & 1u)) {
+            // give the copies in flight a last chance to land, then mark the
+            // tile's outputs: the call has returned long ago
+            for (int m = k; m < nstage && m < k + kDwS; m++)
+                mbar_wait_bounded(&full[m % kDwS], (unsigned)(m / kDwS) & 1u);
+            landed = false;
+            break;
+        }
+        const int nc = min(kDwC, nchan - k * kDwC);
+#pragma unroll 2
+        for (int cc = 0; cc < nc; cc++) {
+            const char* w = reinterpret_cast<const char*>(dsm + (slot * kDwC + cc) * wlen + tid);
+            const uint2* op = reinterpret_cast<const uint2*>(soff + (slot * kDwC + cc) * D);
 #pragma unroll
-            for (int j = 0; j < kDwD; j++) {
-                const int off = dl[j];
+            for (int j4 = 0; j4 < D / 4; j4++) {
+                const uint2 o = op[j4];
+                const unsigned off[4] = {o.x & 0xffffu, o.x >> 16, o.y & 0xffffu, o.y >> 16};
 #pragma unroll
-                for (int q = 0; q < kDdPer; q++) acc[j][q] = __fadd_rn(acc[j][q], w[off + q * kDdThreads]);
+                for (int j = 0; j < 4; j++) {
+                    const float* v = reinterpret_cast<const float*>(w + off[j]);
+#pragma unroll
+                    for (int q = 0; q < P / 2; q++)
+                        acc[4 * j4 + j][q] = add2_rn(acc[4 * j4 + j][q],
+                                                     make_float2(v[2 * q * kDdThreads], v[(2 * q + 1) * kDdThreads]));
+                }
             }
         }
-        __syncthreads();  // buffer buf is refilled by the next iteration's stage
     }
+    const float nan = __int_as_float(0x7fffffff);
 #pragma unroll
-    for (int j = 0; j < kDwD; j++) {
-        if (j < nd) {
+    for (int j = 0; j < D; j++) {
+        if (d0 + j < ndm) {
 #pragma unroll
-            for (int q = 0; q < kDdPer; q++) {
+            for (int q = 0; q < P; q++) {
                 const long long t = t0 + tid + (long long)q * kDdThreads;
-                if (t < nout) out[(long long)(d0 + j) * nout + t] = acc[j][q];
+                if (t < nout)
+                    out[(long long)(d0 + j) * nout + t] = !landed ? nan : (q & 1) ? acc[j][q / 2].y : acc[j][q / 2].x;
             }
         }
     }
+}
+
+// Tables of the windowed form for tiles of D trials; false where the offsets
+// of some tile do not fit (spread in samples, or the ring in shared memory).
+struct DwPlan {
+    int ndtile = 0, wlen = 0;
+    std::vector<long long> start;
+    std::vector<unsigned short> offs;
+};
+
+static size_t dw_smem(int D, int wlen) { return sizeof(float) * kDwS * kDwC * (size_t)wlen + 2 * kDwS * kDwC * D; }
+
+// Widest delay range of a channel within a tile of D trials.
+static int dw_spread(const int* delays, int nchan, int ndm, int D) {
+    int spread = 0;
+    std::vector<int> lo(nchan), hi(nchan);
+    for (int d0 = 0; d0 < ndm; d0 += D) {
+        const int n = std::min(D, ndm - d0);
+        const int* first = delays + (long long)d0 * nchan;
+        std::copy(first, first + nchan, lo.begin());
+        std::copy(first, first + nchan, hi.begin());
+        for (int j = 1; j < n; j++) {
+            const int* row = first + (long long)j * nchan;
+            for (int c = 0; c < nchan; c++) {
+                lo[c] = std::min(lo[c], row[c]);
+                hi[c] = std::max(hi[c], row[c]);
+            }
+        }
+        for (int c = 0; c < nchan; c++) spread = std::max(spread, hi[c] - lo[c]);
+    }
+    return spread;
+}
+
+static void dw_plan(DwPlan& p, const float* in, const int* delays, int nchan, long long nsamp, int ndm, int D,
+                    int wlen) {
+    p.ndtile = (ndm + D - 1) / D;
+    p.wlen = wlen;
+    p.start.resize((size_t)p.ndtile * nchan);
+    const size_t pad = (size_t)(nchan + kDwC - 1) / kDwC * kDwC;  // whole stages: 16-byte rows to copy
+    p.offs.assign(p.ndtile * pad * D, 0);
+    const long long skew = (long long)((reinterpret_cast<uintptr_t>(in) >> 2) & 3);
+    for (int tl = 0; tl < p.ndtile; tl++) {
+        const int n = std::min(D, ndm - tl * D);
+        const int* first = delays + (long long)tl * D * nchan;
+        for (int c = 0; c < nchan; c++) {
+            int lo = first[c];
+            for (int j = 1; j < n; j++) lo = std::min(lo, first[(long long)j * nchan + c]);
+            const long long at = (long long)c * nsamp + lo;
+            const int rem = (int)((at + skew) & 3);
+            p.start[(size_t)tl * nchan + c] = at - rem;
+            unsigned short* o = p.offs.data() + (tl * pad + c) * D;
+            for (int j = 0; j < n; j++) o[j] = (unsigned short)(4 * (first[(long long)j * nchan + c] - lo + rem));
+        }
+    }
+}
+
+template <int D>
+static cudaError_t dw_launch(const DwPlan& p, const float* in, int nchan, long long nsamp, const char* tab, int ndm,
+                             float* out, long long nout, cudaStream_t st) {
+    static std::atomic<unsigned long long> attr{0};
+    int dev = 0;
+    if (attr_pending(attr, &dev)) {
+        cudaError_t e = cudaFuncSetAttribute(k_dedisperse_win<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kDwSmemMax);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_dedisperse_win<D>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+        attr_set(attr, dev);
+    }
+    const long long ntt = (nout + kDwT - 1) / kDwT;
+    const size_t ob = sizeof(long long) * p.start.size();
+    k_dedisperse_win<D><<<(unsigned)(p.ndtile * ntt), kDdThreads, dw_smem(D, p.wlen), st>>>(
+        in, nchan, (long long)nchan * nsamp, reinterpret_cast<const long long*>(tab),
+        reinterpret_cast<const unsigned short*>(tab + ((ob + 15) & ~(size_t)15)), ndm, p.ndtile, p.wlen, out, nout);
+    return cudaGetLastError();
 }
 
 }  // namespace accel
@@ -231,57 +353,34 @@ int accel_dedisperse(const float* filterbank_dev, int nchan, long long nsamp, co
     cudaStream_t st = (cudaStream_t)cuda_stream;
     const long long ntt = (nout + kDdThreads * kDdPer - 1) / (kDdThreads * kDdPer);
     {
-        // windowed kernel: per tile of kDwD trials and channel, the delays
-        // relative to their smallest; the widest window sizes shared memory
-        const int nwt = (ndm + kDwD - 1) / kDwD;
-        std::vector<int> rel((size_t)nwt * nchan * kDwD, 0), wmn((size_t)nwt * nchan, 0);
-        int spread = 0;
-        for (int tl = 0; tl < nwt; tl++)
-            for (int c = 0; c < nchan; c++) {
-                int lo = INT32_MAX, hi = 0;
-                for (int j = 0; j < kDwD && tl * kDwD + j < ndm; j++) {
-                    const int v = delays[(long long)(tl * kDwD + j) * nchan + c];
-                    lo = std::min(lo, v);
-                    hi = std::max(hi, v);
-                }
-                wmn[(size_t)tl * nchan + c] = lo;
-                spread = std::max(spread, hi - lo);
-                for (int j = 0; j < kDwD && tl * kDwD + j < ndm; j++)
-                    rel[((size_t)tl * nchan + c) * kDwD + j] = delays[(long long)(tl * kDwD + j) * nchan + c] - lo;
-            }
-        const int wlen = ((kDdThreads * kDdPer + spread) + 3) & ~3;
-        const size_t smem = sizeof(float) * 2 * kDwC * (size_t)wlen + sizeof(int) * 2 * kDwC * kDwD;
-        if (smem <= 100 * 1024 && (long long)nwt * ntt <= 0x7fffffffLL) {
-            static std::atomic<unsigned long long> attr{0};
-            int dev = 0;
-            cudaError_t e = cudaSuccess;
-            if (attr_pending(attr, &dev)) {
-                e = cudaFuncSetAttribute(k_dedisperse_win, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-                if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute(k_dedisperse_win, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                             cudaSharedmemCarveoutMaxShared);
-                if (e == cudaSuccess) attr_set(attr, dev);
-            }
-            int* d_rel = nullptr;
-            int* d_wmn = nullptr;
-            if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&d_rel), sizeof(int) * rel.size(), st);
-            if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&d_wmn), sizeof(int) * wmn.size(), st);
+        // windowed kernel: the tile height that pads and copies least among
+        // those whose windows fit
+        int D = 0, wlen = 0;
+        double best = 0;
+        for (int d : {16, 8, 4}) {
+            const long long spread = dw_spread(delays, nchan, ndm, d), need = (kDwT + spread + 3 + 3) & ~3LL;
+            const long long nt = (ndm + d - 1) / d;
+            if (4 * (spread + 3) > 65535 || dw_smem(d, (int)need) > kDwSmemMax || nt * ntt > 0x7fffffffLL) continue;
+            const double cost = (double)nt * d * (1.0 + (double)need / ((double)kDwT * d));
+            if (!D || cost < best) D = d, wlen = (int)need, best = cost;
+        }
+        if (D) {
+            DwPlan p;
+            dw_plan(p, filterbank_dev, delays, nchan, nsamp, ndm, D, wlen);
+            const size_t ob = (sizeof(long long) * p.start.size() + 15) & ~(size_t)15;
+            std::vector<char> tab(ob + sizeof(unsigned short) * p.offs.size());
+            std::memcpy(tab.data(), p.start.data(), sizeof(long long) * p.start.size());
+            std::memcpy(tab.data() + ob, p.offs.data(), sizeof(unsigned short) * p.offs.size());
+            char* d_tab = nullptr;
+            cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d_tab), tab.size(), st);
             // from pageable memory: staged before the call returns
+            if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess)
-                e = cudaMemcpyAsync(d_rel, rel.data(), sizeof(int) * rel.size(), cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(d_wmn, wmn.data(), sizeof(int) * wmn.size(), cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) {
-                k_dedisperse_win<<<(unsigned)(nwt * ntt), kDdThreads, smem, st>>>(filterbank_dev, nchan, nsamp, d_rel,
-                                                                                 d_wmn, ndm, nwt, wlen, out_dev, nout);
-                e = cudaGetLastError();
-            }
-            if (d_rel) {
-                const cudaError_t ef = cudaFreeAsync(d_rel, st);
-                if (e == cudaSuccess) e = ef;
-            }
-            if (d_wmn) {
-                const cudaError_t ef = cudaFreeAsync(d_wmn, st);
+                e = D == 16  ? dw_launch<16>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st)
+                    : D == 8 ? dw_launch<8>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st)
+                             : dw_launch<4>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st);
+            if (d_tab) {
+                const cudaError_t ef = cudaFreeAsync(d_tab, st);
                 if (e == cudaSuccess) e = ef;
             }
             if (e != cudaSuccess) return set_error(ACCEL_ERR_CUDA, "accel_dedisperse: %s", cudaGetErrorString(e));
