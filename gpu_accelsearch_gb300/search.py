@@ -48,21 +48,24 @@ CAND_DTYPE = np.dtype([("trial", "i4"), ("step", "i4"), ("r", "f8"), ("z", "f8")
                        ("numharm", "i4"), ("power", "f4"), ("sigma", "f4")])
 
 
-def _native_dtype():
-    """numpy view of N.Candidate (same offsets and size)."""
-    return np.dtype({"names": ["trial", "step", "r", "z", "numharm", "power", "sigma"],
-                     "formats": ["i4", "i4", "f8", "f8", "i4", "f4", "f4"],
-                     "offsets": [N.Candidate.trial.offset, N.Candidate.step.offset,
-                                 N.Candidate.r.offset, N.Candidate.z.offset,
-                                 N.Candidate.numharm.offset, N.Candidate.power.offset,
-                                 N.Candidate.sigma.offset],
-                     "itemsize": C.sizeof(N.Candidate)})
+# numpy views of N.Candidate and N.Optimized (same offsets and sizes)
+_NATIVE = np.dtype({"names": ["trial", "step", "r", "z", "numharm", "power", "sigma"],
+                    "formats": ["i4", "i4", "f8", "f8", "i4", "f4", "f4"],
+                    "offsets": [N.Candidate.trial.offset, N.Candidate.step.offset, N.Candidate.r.offset,
+                                N.Candidate.z.offset, N.Candidate.numharm.offset, N.Candidate.power.offset,
+                                N.Candidate.sigma.offset],
+                    "itemsize": C.sizeof(N.Candidate)})
+_OPT_FIELDS = ("r_grid", "z_grid", "harm_power", "f", "fdot", "period", "pdot")
+_NATIVE_OPT = np.dtype({"names": ["cand", *_OPT_FIELDS],
+                        "formats": [_NATIVE, "f8", "f8", ("f4", (16,)), "f8", "f8", "f8", "f8"],
+                        "offsets": [getattr(N.Optimized, f).offset for f in ("cand", *_OPT_FIELDS)],
+                        "itemsize": C.sizeof(N.Optimized)})
 
 
 def _to_native(cands: np.ndarray):
     buf = (N.Candidate * max(len(cands), 1))()
     if len(cands):
-        view = np.frombuffer(buf, dtype=_native_dtype(), count=len(cands))
+        view = np.frombuffer(buf, dtype=_NATIVE, count=len(cands))
         for f in CAND_DTYPE.names:
             view[f] = cands[f]
     return buf
@@ -71,7 +74,7 @@ def _to_native(cands: np.ndarray):
 def _from_native(buf, n: int) -> np.ndarray:
     out = np.zeros(n, CAND_DTYPE)
     if n:
-        view = np.frombuffer(buf, dtype=_native_dtype(), count=n)
+        view = np.frombuffer(buf, dtype=_NATIVE, count=n)
         for f in CAND_DTYPE.names:
             out[f] = view[f]
     return out
@@ -336,11 +339,12 @@ class AccelSearch:
         N.check(N.lib().accel_optimize_candidates(self._h, nt, ptrs, nbs, rl, tob, src, n, int(refine),
                                                   dst))
         out = np.zeros(n, OPT_DTYPE)
-        for k in range(n):
-            o = dst[k]
-            c = o.cand
-            out[k] = (c.trial, c.step, c.r, c.z, c.numharm, c.power, c.sigma, o.r_grid, o.z_grid,
-                      tuple(o.harm_power), o.f, o.fdot, o.period, o.pdot)
+        if n:
+            view = np.frombuffer(dst, dtype=_NATIVE_OPT, count=n)
+            for f in CAND_DTYPE.names:
+                out[f] = view["cand"][f]
+            for f in _OPT_FIELDS:
+                out[f] = view[f]
         return out
 
     def candidates(self) -> np.ndarray:
@@ -349,17 +353,4 @@ class AccelSearch:
         N.check(L.accel_candidates(self._h, None, 0, C.byref(n)))
         buf = (N.Candidate * max(n.value, 1))()
         N.check(L.accel_candidates(self._h, buf, n.value, C.byref(n)))
-        out = np.zeros(n.value, CAND_DTYPE)
-        raw = np.frombuffer(buf, dtype=np.uint8, count=n.value * C.sizeof(N.Candidate))
-        if n.value:
-            view = np.ndarray(n.value, dtype=np.dtype({
-                "names": ["trial", "step", "r", "z", "numharm", "power", "sigma"],
-                "formats": ["i4", "i4", "f8", "f8", "i4", "f4", "f4"],
-                "offsets": [N.Candidate.trial.offset, N.Candidate.step.offset,
-                            N.Candidate.r.offset, N.Candidate.z.offset,
-                            N.Candidate.numharm.offset, N.Candidate.power.offset,
-                            N.Candidate.sigma.offset],
-                "itemsize": C.sizeof(N.Candidate)}), buffer=raw)
-            for f in CAND_DTYPE.names:
-                out[f] = view[f]
-        return out
+        return _from_native(buf, n.value)

@@ -7,7 +7,7 @@ import ctypes as C
 import numpy as np
 
 from . import native as N
-from .search import CAND_DTYPE
+from .search import _from_native
 
 
 class Server:
@@ -62,11 +62,7 @@ class Server:
         N.check(L.accel_server_result(self._h, rid, None, 0, C.byref(n), C.byref(lat)))
         buf = (N.Candidate * max(n.value, 1))()
         N.check(L.accel_server_result(self._h, rid, buf, n.value, C.byref(n), C.byref(lat)))
-        out = np.zeros(n.value, CAND_DTYPE)
-        for i in range(n.value):
-            c = buf[i]
-            out[i] = (c.trial, c.step, c.r, c.z, c.numharm, c.power, c.sigma)
-        return out, lat.value
+        return _from_native(buf, n.value), lat.value
 
     def timing(self, rid: int) -> dict:
         """Latency breakdown (ms) of a completed request: queue (submission to
