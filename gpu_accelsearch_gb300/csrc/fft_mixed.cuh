@@ -5,7 +5,7 @@
 //   X[k2 + N2 k1] = sum_g W_R^(g k1) (W_M^(g k2) Y_g[k2]),
 //   Y_g = the N2-point transform of x[R n + g], n < N2,
 //
-// so the R transforms Y_g run side by side on the radix-16 Stockham engine
+// so the R transforms Y_g run side by side on the radix-16 engine
 // of fft_smem.cuh (N2/16 threads each, one barrier per pass for all of
 // them), leave their outputs in shared memory, and a last radix-R pass
 // combines them: one butterfly per k2, its R outputs in natural order
@@ -112,6 +112,12 @@ template <int R, int DIR> __device__ __forceinline__ void dft_radix(float2* v) {
     else dft_odd<R, DIR>(v);
 }
 
+// One N2-point buffer: large enough for the transform and for its outputs,
+// one element of padding every 16.
+template <int N2> constexpr int mixed_buffer() {
+    return FftShape<N2>::PADDED > N2 + N2 / 16 ? FftShape<N2>::PADDED : N2 + N2 / 16;
+}
+
 // Thread layout of a short transform.  UNIT threads carry one transform
 // (R groups of N2/16, 16 points each); CTAs of the plane kernel hold U
 // transforms of different rows so that they are whole warps.  For R = 7
@@ -129,7 +135,7 @@ template <int R, int N2> struct MixedShape {
     static constexpr int EXTRA = R == 7 ? 32 : 0;       // threads of the last pass only
     static constexpr int THREADS = FFT_THREADS + EXTRA;
     static_assert(EXTRA == 0 || (U * N2) % THREADS == 0, "the last pass divides evenly");
-    static constexpr int PM2 = FftShape<N2>::PADDED;    // one padded N2-point buffer
+    static constexpr int PM2 = mixed_buffer<N2>();      // one padded N2-point buffer
     // float2 from one group's pair of buffers to the next: with fewer than 16
     // threads per group, the groups sharing a half-warp start T2 float2
     // apart modulo 16 (different banks)
@@ -149,7 +155,7 @@ __device__ __forceinline__ float2 mixed_twiddle(const float2* __restrict__ tw, i
 template <int R, int N2, int DIR, int NB, int GS>
 __device__ __forceinline__ void mixed_last_pass(float2 (&v)[NB][R], const float2* buf,
                                                 const float2* __restrict__ tw, int b) {
-    constexpr int PM2 = FftShape<N2>::PADDED;
+    constexpr int PM2 = mixed_buffer<N2>();
     const float2* p = buf + fft_pad(b);
 #pragma unroll
     for (int g = 0; g < R; g++)

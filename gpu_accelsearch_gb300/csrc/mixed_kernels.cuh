@@ -35,13 +35,14 @@ constexpr int kPrepShortThreads = 256;
 // Dynamic shared memory of the body for R * N2 points: GROUPS padded
 // N2-point buffers.
 ACCEL_HD constexpr size_t prep_short_smem(int R, int N2) {
-    return sizeof(float2) * (size_t)(((R * (N2 / 16) + 31) / 32 * 32) / (N2 / 16)) * (N2 + N2 / 16);
+    return sizeof(float2) * (size_t)(((R * (N2 / 16) + 31) / 32 * 32) / (N2 / 16)) *
+           (N2 + 32);  // mixed_buffer<N2>()
 }
 template <int R, int N2> struct MixedPrepShape {
     static constexpr int T2 = N2 / 16;
     static constexpr int FFT_THREADS = (R * T2 + 31) / 32 * 32;
     static constexpr int GROUPS = FFT_THREADS / T2;
-    static constexpr int PM2 = FftShape<N2>::PADDED;
+    static constexpr int PM2 = mixed_buffer<N2>();
     static constexpr size_t SMEM = prep_short_smem(R, N2);
     static_assert(SMEM == sizeof(float2) * GROUPS * PM2, "layout");
     static_assert(FFT_THREADS <= kPrepShortThreads, "short transform fits the preparation CTA");
@@ -90,7 +91,7 @@ __device__ __forceinline__ void prep_short_body(const PrepArgs& a, const HarmPla
             }
         }
         float2* buf = sm + grp * PM2;
-        fft_run<N2, -1, 1, GroupSync>(x, buf, tw, t, GroupSync{1, S::FFT_THREADS});
+        fft_run<N2, -1, 1, GroupSync, true>(x, buf, tw, t, GroupSync{1, S::FFT_THREADS});
 #pragma unroll
         for (int e = 0; e < 16; e++) buf[fft_pad(t + e * T2)] = x[0][e];
     }
@@ -153,8 +154,8 @@ __global__ void __launch_bounds__(MixedShape<R, N2>::THREADS, MixedShape<R, N2>:
         float2* buf = sm + (u * R + grp) * S::GS;
         // the transforms' barriers: the whole CTA, or (with the extra warp)
         // named barrier 1 over the transforms' threads only
-        if constexpr (S::EXTRA == 0) fft_run<N2, +1, 2>(x, buf, tw, t);
-        else fft_run<N2, +1, 2, GroupSync>(x, buf, tw, t, GroupSync{1, S::FFT_THREADS});
+        if constexpr (S::EXTRA == 0) fft_run<N2, +1, 2, CtaSync, true>(x, buf, tw, t);
+        else fft_run<N2, +1, 2, GroupSync, true>(x, buf, tw, t, GroupSync{1, S::FFT_THREADS});
 #pragma unroll
         for (int e = 0; e < 16; e++) {
             const int i = fft_pad(t + e * T2);

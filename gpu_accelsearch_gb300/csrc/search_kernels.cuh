@@ -139,14 +139,12 @@ __device__ __forceinline__ float2 fold_at(const HarmPlan& H, int z, int half, in
 
 // Row z of a harmonic's plane for one segment, both transforms at once:
 // multiply the segment spectrum D by the folded template, run the inverse
-// transforms and leave p[e] = (power of even output, power of odd output)
-// at m = t + e*M/16.  The templates carry the 1/L normalisation, so |y|^2
-// is the power.
-template <int M, bool F16, bool SPLIT, class Sync = CtaSync>
-__device__ __forceinline__ void plane_powers(const HarmPlan& H, const float2* __restrict__ D, int z,
-                                             float2* sm, const float2* __restrict__ tw, float2 (&p)[16],
-                                             int t, Sync sync = Sync()) {
-    static_assert(!SPLIT, "the sequential layout stores each transform as it completes");
+// transforms and hand out(e, p) the (power of even output, power of odd
+// output) at m = t + e*M/16 as they are formed.  The templates carry the 1/L
+// normalisation, so |y|^2 is the power.
+template <int M, bool F16, class Sync, class Out>
+__device__ __forceinline__ void plane_row(const HarmPlan& H, const float2* __restrict__ D, int z, float2* sm,
+                                          const float2* __restrict__ tw, int t, Sync sync, Out out) {
     constexpr int T = M / 16;
     float2 x[2][16];
 #pragma unroll
@@ -156,11 +154,9 @@ __device__ __forceinline__ void plane_powers(const HarmPlan& H, const float2* __
         x[0][e] = cmul(d, fold_at<M, F16>(H, z, 0, idx));
         x[1][e] = cmul(d, fold_at<M, F16>(H, z, 1, idx));
     }
-    fft_run<M, +1, 2, Sync>(x, sm, tw, t, sync);
-#pragma unroll
-    for (int e = 0; e < 16; e++)
-        p[e] = make_float2(fmaf(x[0][e].x, x[0][e].x, x[0][e].y * x[0][e].y),
-                           fmaf(x[1][e].x, x[1][e].x, x[1][e].y * x[1][e].y));
+    fft_run_to<M, +1, 2, Sync>(x, sm, tw, t, sync, [&](int e, const float2 (&y)[2]) {
+        out(e, make_float2(fmaf(y[0].x, y[0].x, y[0].y * y[0].y), fmaf(y[1].x, y[1].x, y[1].y * y[1].y)));
+    });
 }
 
 // Stage the row's powers for columns [0, wmax) in shared memory (even and
@@ -201,14 +197,12 @@ __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLI
     const int half_w = H.wmax >> 1;
     if constexpr (!SPLIT) {
         // straight from registers: (even, odd) pairs as 8-byte stores
-        float2 p[16];
-        plane_powers<M, F16, false>(H, D, z, reinterpret_cast<float2*>(smem_raw), tw, p, t);
-#pragma unroll
-        for (int e = 0; e < 16; e++) {
-            const int i2 = t + e * T - H.hw0;  // one unsigned compare for 0 <= i2 < half_w
+        const int lo = t - H.hw0;
+        plane_row<M, F16>(H, D, z, reinterpret_cast<float2*>(smem_raw), tw, t, CtaSync(), [&](int e, float2 p) {
+            const int i2 = lo + e * T;  // one unsigned compare for 0 <= i2 < half_w
             // (streaming: the row is next read by the harmonic sum)
-            if ((unsigned)i2 < (unsigned)half_w) __stcs(reinterpret_cast<float2*>(row + 2 * i2), p[e]);
-        }
+            if ((unsigned)i2 < (unsigned)half_w) __stcs(reinterpret_cast<float2*>(row + 2 * i2), p);
+        });
     } else {
         // even transform, then odd, each stored as it completes (a loop, not
         // unrolled, so that nothing of the first stays live in the second)
@@ -220,12 +214,11 @@ __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLI
                 const int idx = t + e * T;
                 x[0][e] = cmul(D[idx], fold_at<M, F16>(H, z, half, idx));
             }
-            fft_run<M, +1, 1>(x, reinterpret_cast<float2*>(smem_raw), tw, t);
-#pragma unroll
-            for (int e = 0; e < 16; e++) {
+            fft_run_to<M, +1, 1>(x, reinterpret_cast<float2*>(smem_raw), tw, t, CtaSync(), [&](int e, const float2 (&y)[1]) {
                 const int i2 = t + e * T - H.hw0;
-                if (i2 >= 0 && i2 < half_w) row[2 * i2 + half] = fmaf(x[0][e].x, x[0][e].x, x[0][e].y * x[0][e].y);
-            }
+                if ((unsigned)i2 < (unsigned)half_w) row[2 * i2 + half] = fmaf(y[0].x, y[0].x, y[0].y * y[0].y);
+            });
+            __syncthreads();  // the buffer is free for the odd transform
         }
     }
 }
@@ -281,8 +274,8 @@ __global__ void __launch_bounds__(PlaneShape<false, M>::THREADS, PlaneShape<fals
     const int z = blockIdx.x;
     const int seg = blockIdx.y;
     float2 p[16];
-    plane_powers<M, F16, false>(H0, a.dbuf + (long long)seg * a.dstride + H0.doff, z,
-                                reinterpret_cast<float2*>(smem_raw), tw, p, (int)threadIdx.x);
+    plane_row<M, F16>(H0, a.dbuf + (long long)seg * a.dstride + H0.doff, z, reinterpret_cast<float2*>(smem_raw), tw,
+                      (int)threadIdx.x, CtaSync(), [&](int e, float2 v) { p[e] = v; });
     const float* pw = stage_row_powers<M>(H0, smem_raw, p, (int)threadIdx.x);
 
     const long long startr = a.segs[seg].startr;

@@ -6,7 +6,7 @@ namespace accel {
 
 template <int MMAX, int NH, bool F16>
 static int step_launch(const StepArgs& a, const float2* tw, cudaStream_t st) {
-    const size_t smem = sizeof(float2) * 2 * FftShape<MMAX>::PADDED;  // >= every tile of the plan
+    constexpr size_t smem = kStepSmem<MMAX>;
     static std::atomic<unsigned long long> attr{0};
     static int per_sm[64] = {0};
     int dev = 0;

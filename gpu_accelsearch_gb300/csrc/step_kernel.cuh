@@ -55,12 +55,28 @@ __device__ __forceinline__ StepItem step_decode(const StepArgs& a, long long it)
     return StepItem{0, (int)b, (int)(q - h0)};
 }
 
+// Transform buffers of a plane item of half length M: MMAX/M rows, two
+// buffers each.
+template <int M, int MMAX> constexpr size_t step_row_bytes() {
+    return sizeof(float2) * (MMAX / M) * 2 * FftShape<M>::PADDED;
+}
+constexpr size_t step_max(size_t a, size_t b) { return a > b ? a : b; }
+// Dynamic shared memory of k_step: the rows of any class side by side (the
+// buffers' padding is per row, so the smallest class needs most), and every
+// tile of the plan.
+template <int MMAX>
+constexpr size_t kStepSmem =
+    step_max(step_max(step_max(step_row_bytes<MMAX, MMAX>(), step_row_bytes<MMAX / 2, MMAX>()),
+                      step_max(step_row_bytes<MMAX / 4, MMAX>(), step_row_bytes<MMAX / 8, MMAX>())),
+             sizeof(float) * kTileSmemFloats);
+
 // Rows [first, first + MMAX/M) of class c, M/16 threads per row.
 template <int M, int MMAX, bool F16>
 __device__ __forceinline__ void step_rows(const StepArgs& a, int c, int seg, int first, unsigned char* smem,
                                           const float2* __restrict__ tw) {
     constexpr int GT = M / 16, G = (MMAX / 16) / GT;
     static_assert(G == 1 || GT % 32 == 0, "named barriers need whole warps");
+    static_assert(step_row_bytes<M, MMAX>() <= kStepSmem<MMAX>, "the rows' buffers fit");
     const int g = threadIdx.x / GT, t = threadIdx.x % GT;
     const int row = first + g;
     if (row >= a.cls_ntpl[c]) return;  // the group's own barrier: nothing else waits for it
@@ -72,15 +88,13 @@ __device__ __forceinline__ void step_rows(const StepArgs& a, int c, int seg, int
     const float2* __restrict__ D = a.dbuf + (long long)seg * a.dstride + H.doff;
     float* out = a.planes + (long long)seg * a.hs.pstride + H.poff + (long long)z * H.prow;
     float2* sm = reinterpret_cast<float2*>(smem) + (size_t)g * 2 * FftShape<M>::PADDED;
-    float2 p[16];
-    if constexpr (G == 1) plane_powers<M, F16, false>(H, D, z, sm, tw, p, t);
-    else plane_powers<M, F16, false, GroupSync>(H, D, z, sm, tw, p, t, GroupSync{1 + g, GT});
-    const int half_w = H.wmax >> 1;
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-        const int i2 = t + e * GT - H.hw0;
-        if (i2 >= 0 && i2 < half_w) *reinterpret_cast<float2*>(out + 2 * i2) = p[e];
-    }
+    const int lo = t - H.hw0, half_w = H.wmax >> 1;
+    auto store = [&](int e, float2 p) {
+        const int i2 = lo + e * GT;
+        if ((unsigned)i2 < (unsigned)half_w) *reinterpret_cast<float2*>(out + 2 * i2) = p;
+    };
+    if constexpr (G == 1) plane_row<M, F16>(H, D, z, sm, tw, t, CtaSync(), store);
+    else plane_row<M, F16>(H, D, z, sm, tw, t, GroupSync{1 + g, GT}, store);
 }
 
 template <int MMAX, bool F16>
