@@ -90,11 +90,12 @@ __global__ void __launch_bounds__(256) k_whiten_scale(const int* __restrict__ bs
 // single-precision rate -- for every level and slope.  Now the median is a
 // bitwise search over keys in registers (counts by redux.sync, stopped when
 // one key is left in the interval) and levels and slopes are computed by one
-// lane per range.  2^21 bins, GB300: medians 55 -> 17 us, scaling 31 -> 13 us
+// lane per range.  2^21 bins, GB300: medians 55 -> 12 us, scaling 31 -> 11 us
 // (cold cache).
 constexpr int kWarpBlockMax = 1024;
 constexpr int kWarpsPerCta = 8;
 constexpr int kScaleRanges = 32;  // write ranges per CTA of the scaling kernel
+constexpr int kScaleWarps = 16;
 
 // Lower median (rank (n - 1) / 2, 0-based) of the warp's n keys, lane l
 // holding keys l, l + 32, ... in key[], unused slots 0xffffffff.
@@ -140,74 +141,81 @@ __device__ __forceinline__ uint32_t warp_median(const uint32_t (&key)[NK], int n
     return __reduce_or_sync(0xffffffffu, mine);
 }
 
-template <int NK>
-__device__ __forceinline__ uint32_t block_median(const float2* __restrict__ spec, int n) {
-    const int lane = threadIdx.x & 31;
-    uint32_t key[NK];
-#pragma unroll
-    for (int j = 0; j < NK; j++) {
-        const int i = lane + 32 * j;
-        key[j] = i < n ? __float_as_uint(power_exact(spec[i])) : 0xffffffffu;
-    }
-    return warp_median<NK>(key, n);
-}
-
 // med[b]: the block's median power (the level's division is left to the
-// scaling kernel).
+// scaling kernel).  NK: registers for the widest block, 32 NK bins; with the
+// widths of one call known, a warp carries no more registers than it needs
+// (32 keys in every warp held the kernel at 32 warps per SM).
+template <int NK>
 __global__ void __launch_bounds__(32 * kWarpsPerCta) k_whiten_medians_warp(const int* __restrict__ bstart,
                                                                            const int* __restrict__ blen,
                                                                            const float2* __restrict__ spec,
                                                                            float* __restrict__ med, int nblocks) {
     const int b = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
     if (b >= nblocks) return;
-    const int s = bstart[b], n = blen[b];
-    // registers for 128 bins (widths at the default cap 200 reach 87 at 2^21
-    // bins), 256, or the largest block
-    const uint32_t k = n <= 128 ? block_median<4>(spec + s, n)
-                     : n <= 256 ? block_median<8>(spec + s, n)
-                                : block_median<kWarpBlockMax / 32>(spec + s, n);
-    if ((threadIdx.x & 31) == 0) med[b] = __uint_as_float(k);
+    const int lane = threadIdx.x & 31, n = blen[b];
+    const float2* __restrict__ s = spec + bstart[b];
+    uint32_t key[NK];
+#pragma unroll
+    for (int j = 0; j < NK; j++) {
+        const int i = lane + 32 * j;
+        key[j] = i < n ? __float_as_uint(power_exact(s[i])) : 0xffffffffu;
+    }
+    const uint32_t k = warp_median<NK>(key, n);
+    if (lane == 0) med[b] = __uint_as_float(k);
+}
+
+template <int NK>
+static void launch_medians(const int* bstart, const int* blen, const float2* spec, float* med, int nblocks,
+                           cudaStream_t st) {
+    k_whiten_medians_warp<NK><<<(nblocks + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, st>>>(
+        bstart, blen, spec, med, nblocks);
 }
 
 // Write ranges as in k_whiten_scale, kScaleRanges per CTA: their starts,
 // levels and slopes by one thread each, then a warp per range.
-__global__ void __launch_bounds__(32 * kWarpsPerCta) k_whiten_scale_warp(const int* __restrict__ bstart,
+__global__ void __launch_bounds__(32 * kScaleWarps) k_whiten_scale_warp(const int* __restrict__ bstart,
                                                                          const int* __restrict__ blen,
                                                                          const float* __restrict__ med, int nb,
                                                                          float2* spec, unsigned numbins,
                                                                          int exact) {
     __shared__ int s_lo[kScaleRanges + 1];
     __shared__ float s_mean[kScaleRanges], s_slope[kScaleRanges];
+    __shared__ double s_level[kScaleRanges + 1];
     const int r0 = blockIdx.x * kScaleRanges, nr = min(kScaleRanges, nb + 1 - r0);
-    auto level = [&](int b) { return (double)med[b] / kLn2w; };
-    if (threadIdx.x <= nr) {
-        const int r = r0 + threadIdx.x;
-        s_lo[threadIdx.x] = r == 0 ? 1 : r <= nb ? bstart[r - 1] + blen[r - 1] / 2 : (int)numbins;
-        if (threadIdx.x < nr) {
-            float mean_old, dslope = 0.f;
-            if (r == 0) {
-                mean_old = (float)level(0);
-                spec[0] = make_float2(1.0f, 0.0f);
-            } else if (r < nb) {
-                mean_old = (float)level(r - 1);
-                dslope = (float)((level(r) - (double)mean_old) / (0.5 * (blen[r - 1] + blen[r])));
+    // levels of blocks first .. first + nr (the tail also looks one block back)
+    const int first = max(0, min(r0 - 1, nb - 2)), i = threadIdx.x;
+    if (i <= kScaleRanges && first + i < nb) s_level[i] = (double)med[first + i] / kLn2w;
+    if (i <= nr) {
+        const int r = r0 + i;
+        s_lo[i] = r == 0 ? 1 : r <= nb ? bstart[r - 1] + blen[r - 1] / 2 : (int)numbins;
+    }
+    __syncthreads();
+    if (i < nr) {
+        const int r = r0 + i;
+        auto level = [&](int b) { return s_level[b - first]; };
+        float mean_old, dslope = 0.f;
+        if (r == 0) {
+            mean_old = (float)level(0);
+            spec[0] = make_float2(1.0f, 0.0f);
+        } else if (r < nb) {
+            mean_old = (float)level(r - 1);
+            dslope = (float)((level(r) - (double)mean_old) / (0.5 * (blen[r - 1] + blen[r])));
+        } else {
+            mean_old = (float)level(nb - 1);
+            if (nb >= 2) {
+                const float mo = (float)level(nb - 2);
+                dslope = (float)((level(nb - 1) - (double)mo) / (0.5 * (blen[nb - 2] + blen[nb - 1])));
             } else {
-                mean_old = (float)level(nb - 1);
-                if (nb >= 2) {
-                    const float mo = (float)level(nb - 2);
-                    dslope = (float)((level(nb - 1) - (double)mo) / (0.5 * (blen[nb - 2] + blen[nb - 1])));
-                } else {
-                    dslope = 1.0f;
-                }
+                dslope = 1.0f;
             }
-            s_mean[threadIdx.x] = mean_old;
-            s_slope[threadIdx.x] = dslope;
         }
+        s_mean[i] = mean_old;
+        s_slope[i] = dslope;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
-    for (int q = threadIdx.x >> 5; q < nr; q += kWarpsPerCta) {
+    for (int q = threadIdx.x >> 5; q < nr; q += kScaleWarps) {
         const unsigned lo = (unsigned)s_lo[q], hi = (unsigned)s_lo[q + 1];
         const float mean_old = s_mean[q], dslope = s_slope[q];
         if (r0 + q == 0) {
@@ -278,11 +286,15 @@ int launch_whiten(const int* d_bstart, const int* d_blen, int nblocks, double* d
                   unsigned numbins, int maxlen, cudaStream_t st, int exact) {
     if (maxlen <= kWarpBlockMax) {
         float* med = reinterpret_cast<float*>(d_med);
-        k_whiten_medians_warp<<<(nblocks + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, st>>>(
-            d_bstart, d_blen, spec, med, nblocks);
+        // widths at the default cap: 78 at 2^18 bins, 87 at 2^21, 99 at 2^24
+        if (maxlen <= 64) launch_medians<2>(d_bstart, d_blen, spec, med, nblocks, st);
+        else if (maxlen <= 96) launch_medians<3>(d_bstart, d_blen, spec, med, nblocks, st);
+        else if (maxlen <= 128) launch_medians<4>(d_bstart, d_blen, spec, med, nblocks, st);
+        else if (maxlen <= 256) launch_medians<8>(d_bstart, d_blen, spec, med, nblocks, st);
+        else launch_medians<kWarpBlockMax / 32>(d_bstart, d_blen, spec, med, nblocks, st);
         if (cudaGetLastError() != cudaSuccess) return -1;
-        k_whiten_scale_warp<<<nblocks / kScaleRanges + 1, 32 * kWarpsPerCta, 0, st>>>(d_bstart, d_blen, med, nblocks,
-                                                                                    spec, numbins, exact);
+        k_whiten_scale_warp<<<nblocks / kScaleRanges + 1, 32 * kScaleWarps, 0, st>>>(d_bstart, d_blen, med, nblocks, spec,
+                                                                                   numbins, exact);
         return cudaGetLastError() == cudaSuccess ? 0 : -1;
     }
     size_t smem = sizeof(uint32_t) * (size_t)maxlen;
