@@ -1,5 +1,5 @@
 // async_copy.cuh -- mbarriers with bounded waits and bulk asynchronous copies
-// (TMA) into shared memory.
+// (TMA) into and out of shared memory.
 #pragma once
 
 #include <cuda.h>
@@ -57,6 +57,21 @@ __device__ __forceinline__ void bulk_copy_g2s(void* sdst, const void* gsrc, unsi
                      smem_addr(sdst)),
                  "l"(gsrc), "r"(bytes), "r"(smem_addr(bar))
                  : "memory");
+}
+
+// bytes (a multiple of 16) from shared to global, both 16-byte aligned; the
+// writers of the shared bytes have fenced (fence_async_proxy) and met at a
+// barrier.  bulk_s2g_wait_read: the issuing thread's copies have read their
+// shared memory (the stores themselves are complete when the kernel is).
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_copy_s2g(void* gdst, const void* ssrc, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(gdst), "r"(smem_addr(ssrc)),
+                 "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void bulk_s2g_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
 }
 
 }  // namespace accel

@@ -177,6 +177,18 @@ __device__ __forceinline__ float* stage_row_powers(const HarmPlan& H, unsigned c
     return pw;
 }
 
+// Rows gathered in shared memory and stored by one bulk copy each, instead of
+// 8-byte stores from the registers.  A store of 256 bytes by a warp takes 6.6
+// wavefronts of the L1 data pipe, a fifth of a 2048-point row's, and the pipe
+// is 92 % busy there; through shared memory the row costs 2 wavefronts for the
+// same bytes, one more barrier pair and the wait of one thread for the copy's
+// reads.  us per segment, stores -> bulk: 2048 points 4.43 -> 4.30 (656 rows),
+// 1024 1.31 -> 1.27, 512 0.64 -> 0.64 (400 rows).  At 4096 points the pipe is
+// 70 % busy and two CTAs per SM hide the wait less: 10.39 -> 10.42; at 8192
+// (one CTA) 13.0 -> 14.5.  A buffer of its own for the row saves a barrier but
+// takes the L1's room: 4.79.
+constexpr bool plane_bulk_rows(int M) { return M == 1024 || M == 2048; }
+
 template <int M, bool F16, bool SPLIT>
 __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLIT, M>::MINB)
     k_plane(const PlaneArgs a, const float2* __restrict__ tw) {
@@ -195,7 +207,36 @@ __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLI
     const float2* __restrict__ D = a.dbuf + (long long)seg * a.dstride + H.doff;
     float* row = a.planes + (long long)seg * a.pstride + H.poff + (long long)z * H.prow;
     const int half_w = H.wmax >> 1;
-    if constexpr (!SPLIT) {
+    if constexpr (!SPLIT && plane_bulk_rows(M)) {
+        const int lo = t - H.hw0;
+        float2 p[16];
+        plane_row<M, F16>(H, D, z, reinterpret_cast<float2*>(smem_raw), tw, t, CtaSync(), [&](int e, float2 v) { p[e] = v; });
+        // (a caller's planes may start on 8 bytes only; the rows are multiples
+        // of 16 bytes apart)
+        const unsigned bytes = (unsigned)(half_w * 8) & ~15u;
+        if ((reinterpret_cast<uintptr_t>(row) & 15) == 0 && bytes > 0) {
+            float2* pw = reinterpret_cast<float2*>(smem_raw);
+            __syncthreads();  // every thread has read its points
+#pragma unroll
+            for (int e = 0; e < 16; e++) {
+                const int i2 = lo + e * T;
+                if ((unsigned)i2 < (unsigned)half_w) pw[i2] = p[e];
+            }
+            fence_async_proxy();
+            __syncthreads();
+            if (t == 0) {
+                bulk_copy_s2g(row, pw, bytes);
+                if (half_w & 1) *reinterpret_cast<float2*>(row + 2 * (half_w - 1)) = pw[half_w - 1];
+                bulk_s2g_wait_read();  // shared memory is free when this returns
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 16; e++) {
+                const int i2 = lo + e * T;
+                if ((unsigned)i2 < (unsigned)half_w) *reinterpret_cast<float2*>(row + 2 * i2) = p[e];
+            }
+        }
+    } else if constexpr (!SPLIT) {
         // straight from registers: (even, odd) pairs as 8-byte stores
         const int lo = t - H.hw0;
         plane_row<M, F16>(H, D, z, reinterpret_cast<float2*>(smem_raw), tw, t, CtaSync(), [&](int e, float2 p) {
