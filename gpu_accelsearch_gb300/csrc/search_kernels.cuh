@@ -184,8 +184,7 @@ __device__ __forceinline__ float* stage_row_powers(const HarmPlan& H, unsigned c
 // same bytes, one more barrier pair and the wait of one thread for the copy's
 // reads.  us per segment, stores -> bulk: 2048 points 4.43 -> 4.30 (656 rows),
 // 1024 1.31 -> 1.27, 512 0.64 -> 0.64 (400 rows).  At 4096 points the pipe is
-// 70 % busy and two CTAs per SM hide the wait less: 10.39 -> 10.42; at 8192
-// (one CTA) 13.0 -> 14.5.  A buffer of its own for the row saves a barrier but
+// 70 % busy and two CTAs per SM hide the wait less: 10.39 -> 10.42.  A buffer of its own for the row saves a barrier but
 // takes the L1's room: 4.79.
 constexpr bool plane_bulk_rows(int M) { return M == 1024 || M == 2048; }
 
@@ -261,6 +260,95 @@ __global__ void __launch_bounds__(PlaneShape<SPLIT, M>::THREADS, PlaneShape<SPLI
             });
             __syncthreads();  // the buffer is free for the odd transform
         }
+    }
+}
+
+// Rows of 8192 points, one transform (half of a row: its even or its odd
+// outputs) per CTA.  With both transforms of a row in one CTA (512 threads, 16
+// points of each) an SM holds a single CTA, whose exchanges (L1-bound) and
+// butterflies (FP32-bound) never overlap, and the transform takes four passes
+// (16 x 16 x 16 x 2) and three exchanges.  Here 256 threads hold 32 points of
+// one transform: two radix-16 butterflies per pass that share their twiddles,
+// and the third pass's two are the inputs of the thread's own radix-2
+// butterflies, so that the third exchange goes, and two CTAs share an SM.  The
+// segment spectrum is loaded by both halves and the powers are stored 4 bytes at
+// a time (the even and the odd ones meet in L2).  Same butterflies, twiddles and
+// order as the transform of fft_smem.cuh, hence the same bits.  300 rows: 13.57
+// -> 12.02 us per segment.  4096 points, which gain no pass, in the same form
+// (128 threads, four CTAs per SM): 10.84 -> 11.86.
+struct PlaneHalf {
+    static constexpr int M = 8192, THREADS = M / 32, PITCH = FftShape<M>::PITCH;
+    static constexpr size_t SMEM = sizeof(float2) * FftShape<M>::PADDED;
+};
+
+template <bool F16>
+__global__ void __launch_bounds__(PlaneHalf::THREADS, 2) k_plane_half(const PlaneArgs a, const float2* __restrict__ tw) {
+    constexpr int M = PlaneHalf::M, T = PlaneHalf::THREADS, PITCH = PlaneHalf::PITCH;
+    constexpr bool PK = M < 8192;  // as fft_smem.cuh's transform
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    const int item = blockIdx.y;
+    int hi = 0;
+#pragma unroll 1
+    while (hi + 1 < a.nh && item >= a.h[hi + 1].zbase) hi++;
+    const HarmPlan& H = a.h[hi];
+    const int z = item - H.zbase;
+    // the two halves of a row side by side, then the segments (as in k_plane)
+    const int seg = blockIdx.x >> 1, half = blockIdx.x & 1;
+    const int t = threadIdx.x;
+    const float2* __restrict__ D = a.dbuf + (long long)seg * a.dstride + H.doff;
+    float* row = a.planes + (long long)seg * a.pstride + H.poff + (long long)z * H.prow + half;
+    const int half_w = H.wmax >> 1;
+    float2 x[2][16];
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int e = 0; e < 16; e++) {
+            const int n = t + T * j + 2 * T * e;
+            x[j][e] = cmul(D[n], fold_at<M, F16>(H, z, half, n));
+        }
+    // first pass: blocks k1, positions n1 + 32 n2 of a block
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        dft<16, 1, PK>(x[j]);
+#pragma unroll
+        for (int r = 0; r < 16; r++) sm[t + T * j + r * PITCH] = x[j][r];
+    }
+    __syncthreads();
+    // second: k1 = t / 16, n1 = t % 16 and 16 more
+    float2* p = sm + (t >> 4) * PITCH + (t & 15);
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int r = 0; r < 16; r++) x[j][r] = p[16 * j + 32 * r];
+    apply_tw16_full256<1, 2>(x, tw, t >> 4);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        dft<16, 1, PK>(x[j]);
+#pragma unroll
+        for (int r = 0; r < 16; r++) p[16 * j + 32 * r] = x[j][r];
+    }
+    const Tw16 p2 = load_tw16<1>(tw, t, M / 2);
+    __syncthreads();
+    // third and last: k1 = t % 16, k2 = t / 16, all 32 positions of the pair
+    const float4* q = reinterpret_cast<const float4*>(sm + (t & 15) * PITCH + 32 * (t >> 4));
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const float4 v = q[r];
+        x[0][r] = make_float2(v.x, v.y);
+        x[1][r] = make_float2(v.z, v.w);
+    }
+    apply_tw16<2>(x, p2);
+    dft<16, 1, PK>(x[0]);
+    dft<16, 1, PK>(x[1]);
+    const int lo = t - H.hw0;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const float2 v = cmul(x[1][r], twid<1>(tw, t + T * r));
+        const float2 y0 = cadd(x[0][r], v), y1 = csub(x[0][r], v);
+        const int i0 = lo + T * r, i1 = i0 + M / 2;
+        if ((unsigned)i0 < (unsigned)half_w) __stcs(row + 2 * i0, fmaf(y0.x, y0.x, y0.y * y0.y));
+        if ((unsigned)i1 < (unsigned)half_w) __stcs(row + 2 * i1, fmaf(y1.x, y1.x, y1.y * y1.y));
     }
 }
 
@@ -915,11 +1003,33 @@ static int plane_m(const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t 
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+template <bool F16>
+static int plane_half(const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t st) {
+    static std::atomic<unsigned long long> attr{0};
+    int dev = 0;
+    if (attr_pending(attr, &dev)) {
+        if (cudaFuncSetAttribute(k_plane_half<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)PlaneHalf::SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_plane_half<F16>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 carveout_for((const void*)k_plane_half<F16>, PlaneHalf::THREADS,
+                                              PlaneHalf::SMEM)) != cudaSuccess)
+            return -1;
+        attr_set(attr, dev);
+    }
+    k_plane_half<F16><<<dim3(2 * nseg, a.ntpl), PlaneHalf::THREADS, PlaneHalf::SMEM, st>>>(a, tw);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
 template <int M>
 static int plane_dispatch(const PlaneArgs& a, int nseg, const float2* tw, cudaStream_t st) {
     const bool h = a.use_fp16 != 0, sp = a.split != 0;
-    if (h) return sp ? plane_m<M, true, true>(a, nseg, tw, st) : plane_m<M, true, false>(a, nseg, tw, st);
-    return sp ? plane_m<M, false, true>(a, nseg, tw, st) : plane_m<M, false, false>(a, nseg, tw, st);
+    if constexpr (M == PlaneHalf::M) {
+        if (h) return sp ? plane_m<M, true, true>(a, nseg, tw, st) : plane_half<true>(a, nseg, tw, st);
+        return sp ? plane_m<M, false, true>(a, nseg, tw, st) : plane_half<false>(a, nseg, tw, st);
+    } else {
+        if (h) return sp ? plane_m<M, true, true>(a, nseg, tw, st) : plane_m<M, true, false>(a, nseg, tw, st);
+        return sp ? plane_m<M, false, true>(a, nseg, tw, st) : plane_m<M, false, false>(a, nseg, tw, st);
+    }
 }
 
 template <int M, bool F16>
