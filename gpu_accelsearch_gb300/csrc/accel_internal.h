@@ -162,8 +162,8 @@ inline void attr_set(std::atomic<unsigned long long>& done, int dev) {
 // The smallest shared-memory carveout (percent of the SM's shared memory)
 // that holds as many CTAs of `kernel` as its registers and threads allow:
 // the rest of the unified L1/shared array stays L1 for the kernel's global
-// loads (the plane kernel: 2 CTAs of 70 KB take the 164 KB configuration,
-// leaving 92 KB of L1 instead of 28 KB at the largest carveout).
+// loads (the plane kernel: 2 CTAs of 66 KB take the 132 KB configuration,
+// leaving 124 KB of L1 instead of 28 KB at the largest carveout).
 inline int carveout_for(const void* kernel, int threads, size_t dyn_smem) {
     cudaFuncAttributes fa{};
     int dev = 0, smem_sm = 0, reserved = 0, regs_sm = 0, thr_sm = 0;
