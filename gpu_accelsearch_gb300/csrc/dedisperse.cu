@@ -129,11 +129,31 @@ __device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
     return r;
 }
 
+// The tile's outputs of one thread, each sample read from global memory:
+// start and offs are the tile's, t the thread's first output sample.
+template <int D>
+__device__ __noinline__ void dw_tile_from_global(const float* __restrict__ in, int nchan,
+                                                 const long long* __restrict__ start,
+                                                 const unsigned short* __restrict__ offs, long long t, int nd,
+                                                 float* __restrict__ out, long long nout) {
+#pragma unroll 1
+    for (int j = 0; j < nd; j++)
+#pragma unroll 1
+        for (int q = 0; q < kDdPer; q++) {
+            const long long tq = t + (long long)q * kDdThreads;
+            if (tq >= nout) break;
+            float s = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < nchan; c++) s = __fadd_rn(s, __ldg(in + start[c] + offs[c * D + j] / 4 + tq));
+            out[(long long)j * nout + tq] = s;
+        }
+}
+
 template <int D>
 __global__ void __launch_bounds__(kDdThreads, 2)
     k_dedisperse_win(const float* __restrict__ in, int nchan, long long total, const long long* __restrict__ start,
                      const unsigned short* __restrict__ offs, int ndm, int ndtile, int wlen, float* __restrict__ out,
-                     long long nout) {
+                     long long nout, unsigned test_extra_tx) {
     constexpr int P = kDdPer;
     extern __shared__ __align__(128) float dsm[];  // [kDwS][kDwC][wlen] windows, then [kDwS][kDwC][D] offsets
     unsigned short* soff = reinterpret_cast<unsigned short*>(dsm + kDwS * kDwC * wlen);
@@ -167,7 +187,7 @@ __global__ void __launch_bounds__(kDdThreads, 2)
             // before the bulk writes
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             constexpr unsigned ob = 2u * D * kDwC;
-            mbar_arrive_expect_tx(&full[slot], bytes + ob);
+            mbar_arrive_expect_tx(&full[slot], bytes + ob + test_extra_tx);
             bulk_copy_g2s(soff + slot * kDwC * D, offs + ((long long)tile * nstage + k) * kDwC * D, ob, &full[slot]);
             for (int cc = 0; cc < nc; cc++) {
                 const long long at = st[cc] + t0;
@@ -182,22 +202,18 @@ __global__ void __launch_bounds__(kDdThreads, 2)
 #pragma unroll
         for (int q = 0; q < P / 2; q++) acc[j][q] = make_float2(0.f, 0.f);
     for (int k = 0; k < kDwS - 1 && k < nstage; k++) fill(k);
-    bool landed = true;
+    int landed = 1;
+    int k = 0;
 #pragma unroll 1
-    for (int k = 0; k < nstage; k++) {
+    for (; k < nstage; k++) {
         const int slot = k % kDwS;
-        // everyone is done with stage k - 1 (its slot is refilled now) and
-        // sees the samples copied one by one for stage k
-        __syncthreads();
+        // everyone is done with stage k - 1 (its slot is refilled now), sees
+        // the samples copied one by one for stage k, and agrees on whether
+        // stage k - 1 had landed: either all go on or all leave here
+        if (!__syncthreads_and(landed)) break;
         if (k + kDwS - 1 < nstage) fill(k + kDwS - 1);
-        if (!mbar_wait_bounded(&full[slot], (unsigned)(k / kDwS) & 1u)) {
-            // give the copies in flight a last chance to land, then mark the
-            // tile's outputs: the call has returned long ago
-            for (int m = k; m < nstage && m < k + kDwS; m++)
-                mbar_wait_bounded(&full[m % kDwS], (unsigned)(m / kDwS) & 1u);
-            landed = false;
-            break;
-        }
+        landed = mbar_wait_bounded(&full[slot], (unsigned)(k / kDwS) & 1u);
+        if (!landed) continue;
         const int nc = min(kDwC, nchan - k * kDwC);
 #pragma unroll 2
         for (int cc = 0; cc < nc; cc++) {
@@ -218,15 +234,25 @@ __global__ void __launch_bounds__(kDdThreads, 2)
             }
         }
     }
-    const float nan = __int_as_float(0x7fffffff);
+    if (!__syncthreads_and(landed)) {
+        // A copy did not land within the wait's limit (stage k - 1; up to
+        // kDwS - 1 later ones are in flight: a last chance for all of them).
+        // The call has returned long ago and has no status left to give, so
+        // the tile is summed from global memory instead: the same samples in
+        // the same order.
+        for (int m = k - 1; m < nstage && m < k - 1 + kDwS; m++)
+            mbar_wait_bounded(&full[m % kDwS], (unsigned)(m / kDwS) & 1u);
+        dw_tile_from_global<D>(in, nchan, start + (long long)tile * nchan, offs + (long long)tile * nstage * kDwC * D,
+                               t0 + tid, min(D, ndm - d0), out + (long long)d0 * nout, nout);
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < D; j++) {
         if (d0 + j < ndm) {
 #pragma unroll
             for (int q = 0; q < P; q++) {
                 const long long t = t0 + tid + (long long)q * kDdThreads;
-                if (t < nout)
-                    out[(long long)(d0 + j) * nout + t] = !landed ? nan : (q & 1) ? acc[j][q / 2].y : acc[j][q / 2].x;
+                if (t < nout) out[(long long)(d0 + j) * nout + t] = (q & 1) ? acc[j][q / 2].y : acc[j][q / 2].x;
             }
         }
     }
@@ -288,7 +314,7 @@ static void dw_plan(DwPlan& p, const float* in, const int* delays, int nchan, lo
 
 template <int D>
 static cudaError_t dw_launch(const DwPlan& p, const float* in, int nchan, long long nsamp, const char* tab, int ndm,
-                             float* out, long long nout, cudaStream_t st) {
+                             float* out, long long nout, bool wait_test, cudaStream_t st) {
     static std::atomic<unsigned long long> attr{0};
     int dev = 0;
     if (attr_pending(attr, &dev)) {
@@ -304,7 +330,8 @@ static cudaError_t dw_launch(const DwPlan& p, const float* in, int nchan, long l
     const size_t ob = sizeof(long long) * p.start.size();
     k_dedisperse_win<D><<<(unsigned)(p.ndtile * ntt), kDdThreads, dw_smem(D, p.wlen), st>>>(
         in, nchan, (long long)nchan * nsamp, reinterpret_cast<const long long*>(tab),
-        reinterpret_cast<const unsigned short*>(tab + ((ob + 15) & ~(size_t)15)), ndm, p.ndtile, p.wlen, out, nout);
+        reinterpret_cast<const unsigned short*>(tab + ((ob + 15) & ~(size_t)15)), ndm, p.ndtile, p.wlen, out, nout,
+        wait_test ? 16u : 0u);
     return cudaGetLastError();
 }
 
@@ -312,33 +339,8 @@ static cudaError_t dw_launch(const DwPlan& p, const float* in, int nchan, long l
 
 using namespace accel;
 
-extern "C" {
-
-int accel_dedisperse_delays(int nchan, double f_top_mhz, double chan_bw_mhz, double tsamp, const float* dms,
-                            int ndm, int* delays, int* max_delay) {
-    if (nchan < 1 || ndm < 1 || !dms || !delays || !(tsamp > 0.0) || !(f_top_mhz > 0.0) || chan_bw_mhz == 0.0)
-        return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: bad argument");
-    const double f_last = f_top_mhz + (nchan - 1) * chan_bw_mhz;
-    if (!(f_last > 0.0)) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: channel frequency <= 0");
-    const double f_ref = std::max(f_top_mhz, f_last);
-    const double inv_ref2 = 1.0 / (f_ref * f_ref);
-    int mx = 0;
-    for (int d = 0; d < ndm; d++) {
-        if (!(dms[d] >= 0.0f)) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: DM %d < 0", d);
-        for (int c = 0; c < nchan; c++) {
-            const double f = f_top_mhz + c * chan_bw_mhz;
-            const double v = std::floor(kDispConst * (double)dms[d] * (1.0 / (f * f) - inv_ref2) / tsamp + 0.5);
-            if (v > 2147483647.0) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: delay overflow");
-            delays[(long long)d * nchan + c] = (int)v;
-            mx = std::max(mx, (int)v);
-        }
-    }
-    if (max_delay) *max_delay = mx;
-    return ACCEL_OK;
-}
-
-int accel_dedisperse(const float* filterbank_dev, int nchan, long long nsamp, const int* delays, int ndm,
-                     float* out_dev, long long nout, void* cuda_stream) {
+static int dedisperse(const float* filterbank_dev, int nchan, long long nsamp, const int* delays, int ndm,
+                      float* out_dev, long long nout, bool wait_test, void* cuda_stream) {
     if (!filterbank_dev || !out_dev || !delays || nchan < 1 || ndm < 1 || nsamp < 1 || nout < 1)
         return set_error(ACCEL_ERR_INVALID, "accel_dedisperse: bad argument");
     const long long nd = (long long)ndm * nchan;
@@ -376,9 +378,9 @@ int accel_dedisperse(const float* filterbank_dev, int nchan, long long nsamp, co
             // from pageable memory: staged before the call returns
             if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess)
-                e = D == 16  ? dw_launch<16>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st)
-                    : D == 8 ? dw_launch<8>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st)
-                             : dw_launch<4>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, st);
+                e = D == 16  ? dw_launch<16>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, wait_test, st)
+                    : D == 8 ? dw_launch<8>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, wait_test, st)
+                             : dw_launch<4>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, wait_test, st);
             if (d_tab) {
                 const cudaError_t ef = cudaFreeAsync(d_tab, st);
                 if (e == cudaSuccess) e = ef;
@@ -410,6 +412,41 @@ int accel_dedisperse(const float* filterbank_dev, int nchan, long long nsamp, co
     if (e == cudaSuccess) e = ef;
     if (e != cudaSuccess) return set_error(ACCEL_ERR_CUDA, "accel_dedisperse: %s", cudaGetErrorString(e));
     return ACCEL_OK;
+}
+
+extern "C" {
+
+int accel_dedisperse_delays(int nchan, double f_top_mhz, double chan_bw_mhz, double tsamp, const float* dms,
+                            int ndm, int* delays, int* max_delay) {
+    if (nchan < 1 || ndm < 1 || !dms || !delays || !(tsamp > 0.0) || !(f_top_mhz > 0.0) || chan_bw_mhz == 0.0)
+        return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: bad argument");
+    const double f_last = f_top_mhz + (nchan - 1) * chan_bw_mhz;
+    if (!(f_last > 0.0)) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: channel frequency <= 0");
+    const double f_ref = std::max(f_top_mhz, f_last);
+    const double inv_ref2 = 1.0 / (f_ref * f_ref);
+    int mx = 0;
+    for (int d = 0; d < ndm; d++) {
+        if (!(dms[d] >= 0.0f)) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: DM %d < 0", d);
+        for (int c = 0; c < nchan; c++) {
+            const double f = f_top_mhz + c * chan_bw_mhz;
+            const double v = std::floor(kDispConst * (double)dms[d] * (1.0 / (f * f) - inv_ref2) / tsamp + 0.5);
+            if (v > 2147483647.0) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse_delays: delay overflow");
+            delays[(long long)d * nchan + c] = (int)v;
+            mx = std::max(mx, (int)v);
+        }
+    }
+    if (max_delay) *max_delay = mx;
+    return ACCEL_OK;
+}
+
+int accel_dedisperse(const float* filterbank_dev, int nchan, long long nsamp, const int* delays, int ndm,
+                     float* out_dev, long long nout, void* cuda_stream) {
+    return dedisperse(filterbank_dev, nchan, nsamp, delays, ndm, out_dev, nout, false, cuda_stream);
+}
+
+int accel_dedisperse_wait_test(const float* filterbank_dev, int nchan, long long nsamp, const int* delays, int ndm,
+                               float* out_dev, long long nout, void* cuda_stream) {
+    return dedisperse(filterbank_dev, nchan, nsamp, delays, ndm, out_dev, nout, true, cuda_stream);
 }
 
 }  // extern "C"

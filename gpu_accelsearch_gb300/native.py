@@ -156,6 +156,8 @@ SIGNATURES = {
                                           C.POINTER(C.c_float), C.c_int, C.POINTER(C.c_int),
                                           C.POINTER(C.c_int)]),
     "accel_dedisperse": (C.c_int, [_vp, C.c_int, _ll, C.POINTER(C.c_int), C.c_int, _vp, _ll, _vp]),
+    "accel_dedisperse_wait_test": (C.c_int, [_vp, C.c_int, _ll, C.POINTER(C.c_int), C.c_int, _vp, _ll,
+                                             _vp]),
     "accel_read_filterbank": (C.c_int, [C.c_char_p, C.POINTER(FilterbankInfo),
                                         C.POINTER(C.POINTER(C.c_float))]),
     "accel_free_host": (None, [_vp]),

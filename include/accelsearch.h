@@ -415,9 +415,16 @@ int  accel_dedisperse_delays(int nchan, double f_top_mhz, double chan_bw_mhz, do
  * delays: int[ndm][nchan] in host memory; out_dev: float[ndm][nout] on the
  * device, nout <= nsamp - max delay.  Runs on cuda_stream (NULL: the legacy
  * default stream); each DM trial row of out_dev is a series accel_search
- * takes with series_on_device = 1. */
+ * takes with series_on_device = 1.  The call does not wait for its kernel;
+ * a tile whose copies into shared memory fail to land within their bounded
+ * wait is summed from global memory, with the same result. */
 int  accel_dedisperse(const float *filterbank_dev, int nchan, long long nsamp, const int *delays,
                       int ndm, float *out_dev, long long nout, void *cuda_stream);
+/* Failure-detection test: the same call with every such wait made to run out
+ * (about 0.1 s per resident tile). */
+int  accel_dedisperse_wait_test(const float *filterbank_dev, int nchan, long long nsamp,
+                                const int *delays, int ndm, float *out_dev, long long nout,
+                                void *cuda_stream);
 
 /* SIGPROC filterbank reader (host only; the reference reads dedispersed
  * .dat series only, bpd_data.c:9-75, and no function of it is replaced):
