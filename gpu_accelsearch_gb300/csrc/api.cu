@@ -538,6 +538,16 @@ int do_rfft(accel_ctx* c, const float* series, long long n, float2* spec) {
     return ACCEL_OK;
 }
 
+// Work of the caller's call is in flight when the call returns: what
+// accel_destroy waits for.  (Work recorded into a caller's graph is the
+// graph's.)
+void mark_async(accel_ctx* c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        cudaEventRecord(c->ev_async, c->stream) == cudaSuccess)
+        c->async_issued = true;
+}
+
 // Launch one group of nseg prepared segment descriptors (device array).
 // fused: the fundamental's plane is not stored; k_fund_sum adds the
 // sub-harmonic planes to it row by row (the search path).  Otherwise every
@@ -1035,6 +1045,9 @@ int run_search(accel_ctx* c, int ntrials, float2* const* spec, const long long* 
 void free_ctx(accel_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
+    // memory that came from the stream-ordered allocator is freed below
+    // without waiting for its users
+    if (c->async_issued) cudaEventSynchronize(c->ev_async);
     c->r2c.clear();
     for (auto& e : c->pending) {
         cudaEventDestroy(e.a);
@@ -1043,6 +1056,7 @@ void free_ctx(accel_ctx* c) {
     for (auto e : c->evpool) cudaEventDestroy(e);
     if (c->ev_begin) cudaEventDestroy(c->ev_begin);
     if (c->ev_end) cudaEventDestroy(c->ev_end);
+    if (c->ev_async) cudaEventDestroy(c->ev_async);
     for (auto& kv : c->wplans) {
         cudaFree(kv.second.d_start);
         cudaFree(kv.second.d_len);
@@ -1152,7 +1166,8 @@ int accel_create(const accel_config* cfg, accel_ctx** out) {
         if (e != cudaSuccess) rc = set_err(ACCEL_ERR_NOMEM, "twiddles: %s", cudaGetErrorString(e));
         else if (launch_twiddles(c->tw, c->stream) != 0) rc = set_err(ACCEL_ERR_CUDA, "twiddle launch");
     }
-    if (!rc && (cudaEventCreate(&c->ev_begin) != cudaSuccess || cudaEventCreate(&c->ev_end) != cudaSuccess))
+    if (!rc && (cudaEventCreate(&c->ev_begin) != cudaSuccess || cudaEventCreate(&c->ev_end) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->ev_async, cudaEventDisableTiming) != cudaSuccess))
         rc = set_err(ACCEL_ERR_CUDA, "event creation failed");
     if (!rc) rc = build_bank(c);
     if (!rc) rc = build_plan(c);
@@ -1362,7 +1377,9 @@ int accel_whiten(accel_ctx* c, accel_complex* spec, long long numbins) {
                        kMaxWhitenBins);
     int rc = ensure_device(c);
     if (rc) return rc;
-    return do_whiten(c, reinterpret_cast<float2*>(spec), (unsigned)numbins);
+    rc = do_whiten(c, reinterpret_cast<float2*>(spec), (unsigned)numbins);
+    mark_async(c);
+    return rc;
 }
 
 int accel_whiten_blocks(long long numbins, int initbuf, int maxbuf, int* start, int* len, long long cap,
@@ -1380,7 +1397,9 @@ int accel_rfft(accel_ctx* c, const float* series, long long n, accel_complex* sp
     if (!c || !series || !spec || n < 2 || (n & 1)) return set_err(ACCEL_ERR_INVALID, "bad argument");
     int rc = ensure_device(c);
     if (rc) return rc;
-    return do_rfft(c, series, n, reinterpret_cast<float2*>(spec));
+    rc = do_rfft(c, series, n, reinterpret_cast<float2*>(spec));
+    mark_async(c);
+    return rc;
 }
 
 int accel_search(accel_ctx* c, int ntrials, const float* const* series, const long long* nsamples,
@@ -1466,11 +1485,15 @@ int accel_search(accel_ctx* c, int ntrials, const float* const* series, const lo
     c->last_trials = ntrials;
     if (on_device) {
         for (int i = 0; i < ntrials && !rc; i++) rc = prepare(i);
-        if (rc) return rc;
+        if (rc) {
+            mark_async(c);
+            return rc;
+        }
         rc = run_search(c, ntrials, specs.data(), nb.data(), rlo.data(), nullptr);
     } else {
         rc = run_search(c, ntrials, specs.data(), nb.data(), rlo.data(), prepare);
     }
+    if (rc) mark_async(c);  // a search that failed may not have waited for its work
     if (ncand) *ncand = (long long)c->last_raw;
     return rc;
 }
