@@ -14,11 +14,14 @@
 // points.  Every phase is a multiple of pi/K reduced exactly to r in
 // [0, 2K) (m^2 mod 2K in integers) and evaluated as the product of two table
 // entries, exp(i pi q S/K) exp(i pi t/K) with r = q S + t, S ~ sqrt(2K),
-// each kept as the sum of two floats and multiplied with the products'
-// rounding errors carried along: within 0.51 units in the last place of the
-// float result, like a double-precision product rounded once, without
-// double-precision operations (1/64 of the FP32 rate: the four per bin alone
-// held the unpacking kernel at 15 us for K = 2^21, now 8.5).  The N/2 + 1 bins follow from the
+// and gives the double-precision product of the two rounded once to float.
+// The double-precision operations (1/64 of the FP32 rate: the four per bin
+// alone held the unpacking kernel at 15 us for K = 2^21, now 8.5) are done only
+// where they can matter: the entries are kept as sums of two floats as well,
+// multiplied with the products' rounding errors carried along, and only where
+// that result lies so close to the middle of two floats that its own error
+// could decide (3 in 100000) is the double product formed.  The N/2 + 1 bins
+// follow from the
 // transforms of the even and odd samples, E[k] = (Z[k] + conj Z[K-k]) / 2
 // and O[k] = (Z[k] - conj Z[K-k]) / (2i):
 //     X[k] = E[k] + exp(-2 pi i k / N) O[k],   k = 0 .. K   (Z[K] = Z[0]).
@@ -49,9 +52,9 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
 }
 
 // Phase tables of exp(i pi r / K): entry t < S is exp(i pi t / K), entry
-// S + q is exp(i pi q S / K) for q < ceil(2K/S); each component as a float
-// (x, y) and what that rounding left (z, w).
-__global__ void k_phase_tables(float4* __restrict__ tab, long long K, int S, int nq) {
+// S + q is exp(i pi q S / K) for q < ceil(2K/S); in double, and each component
+// as a float (x, y) and what that rounding left (z, w).
+__global__ void k_phase_tables(float4* __restrict__ tab, double2* __restrict__ dbl, long long K, int S, int nq) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S + nq) return;
     double s, c;
@@ -59,25 +62,42 @@ __global__ void k_phase_tables(float4* __restrict__ tab, long long K, int S, int
     else sincospi((double)(i - S) * (double)S / (double)K, &s, &c);
     const float ch = (float)c, sh = (float)s;
     tab[i] = make_float4(ch, sh, (float)(c - (double)ch), (float)(s - (double)sh));
+    dbl[i] = make_double2(c, s);
 }
 
 struct Phase {
     const float4* tab;
+    const double2* dbl;
     unsigned S, shift;  // S = 2^shift
-    // exp(i pi r / K) for 0 <= r < 2K, rounded (almost always) once
+    // exp(i pi r / K) for 0 <= r < 2K: the double product, rounded once
     __device__ __forceinline__ float2 operator()(unsigned r) const {
+        bool sure;
+        const float2 v = fast(r, sure);
+        return sure ? v : exact(r);
+    }
+    // without double precision: the same value wherever sure is set
+    __device__ __forceinline__ float2 fast(unsigned r, bool& sure) const {
         const float4 a = __ldg(tab + S + (r >> shift)), b = __ldg(tab + (r & (S - 1)));
-        return make_float2(diff_of_products(a.x, a.z, b.x, b.z, a.y, a.w, b.y, b.w),
-                           diff_of_products(a.x, a.z, b.y, b.w, -a.y, -a.w, b.x, b.z));
+        sure = true;
+        return make_float2(diff_of_products(a.x, a.z, b.x, b.z, a.y, a.w, b.y, b.w, sure),
+                           diff_of_products(a.x, a.z, b.y, b.w, -a.y, -a.w, b.x, b.z, sure));
+    }
+    __device__ __forceinline__ float2 exact(unsigned r) const {
+        const double2 a = __ldg(dbl + S + (r >> shift)), b = __ldg(dbl + (r & (S - 1)));
+        return make_float2((float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x));
     }
     // the same with the plain float product (error about 1e-7)
     __device__ __forceinline__ float2 f(unsigned r) const {
         const float4 a = __ldg(tab + S + (r >> shift)), b = __ldg(tab + (r & (S - 1)));
         return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
     }
-    // (p + pl)(q + ql) - (u + ul)(v + vl) of two-float numbers
+    // (p + pl)(q + ql) - (u + ul)(v + vl) of two-float numbers.  The sum before
+    // the last rounding is within 7 2^-48 of the exact value (entries 2^-48,
+    // the neglected low product 2^-49, the additions 5.5 2^-48; 2^-45.9 is the
+    // largest measured): where 2^-44 either way rounds alike, so does the
+    // double product; elsewhere sure is cleared.
     static __device__ __forceinline__ float diff_of_products(float p, float pl, float q, float ql, float u, float ul,
-                                                             float v, float vl) {
+                                                             float v, float vl, bool& sure) {
         const float m = __fmul_rn(p, q), n = __fmul_rn(u, v);
         const float me = __fmaf_rn(p, q, -m), ne = __fmaf_rn(u, v, -n);  // exact: m + me = p q
         const float d = __fsub_rn(m, n), t = __fsub_rn(d, m);
@@ -87,6 +107,8 @@ struct Phase {
         low = __fmaf_rn(pl, q, low);
         low = __fmaf_rn(-u, vl, low);
         low = __fmaf_rn(-ul, v, low);
+        constexpr float kTol = 1.0f / (1ull << 44);
+        sure = sure && __fadd_rn(d, __fadd_rn(low, kTol)) == __fadd_rn(d, __fsub_rn(low, kTol));
         return __fadd_rn(d, low);
     }
 };
@@ -163,12 +185,18 @@ __device__ __forceinline__ void unpack_pair(float2* __restrict__ X, long long K,
     // E = (Z[k] + conj Z[K-k]) / 2, O = (Z[k] - conj Z[K-k]) / (2i)
     const float2 e = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y - zc.y));
     const float2 o = make_float2(0.5f * (zk.y + zc.y), -0.5f * (zk.x - zc.x));
-    const float2 v = ph((unsigned)k);             // exp(+i pi k / K) = exp(2 pi i k / N)
-    const float2 t = make_float2(v.x, -v.y);      // exp(-2 pi i k / N)
-    const float2 to = make_float2(t.x * o.x - t.y * o.y, t.x * o.y + t.y * o.x);
-    X[k] = make_float2(e.x + to.x, e.y + to.y);
-    // X[K-k] = conj(E) - conj(t) conj(O) = conj(E - t O)
-    if (2 * k != K) X[K - k] = make_float2(e.x - to.x, -(e.y - to.y));
+    auto put = [&](float2 v) {                    // v = exp(+i pi k / K) = exp(2 pi i k / N)
+        const float2 t = make_float2(v.x, -v.y);  // exp(-2 pi i k / N)
+        const float2 to = make_float2(t.x * o.x - t.y * o.y, t.x * o.y + t.y * o.x);
+        X[k] = make_float2(e.x + to.x, e.y + to.y);
+        // X[K-k] = conj(E) - conj(t) conj(O) = conj(E - t O)
+        if (2 * k != K) X[K - k] = make_float2(e.x - to.x, -(e.y - to.y));
+    };
+    // (the rare other rounding stored afterwards: taken before, the branch
+    // stood between the loop's loads: K = 2^21 took 6 us longer)
+    bool sure;
+    put(ph.fast((unsigned)k, sure));
+    if (!sure) put(ph.exact((unsigned)k));
 }
 
 // In place over X[0 .. K]: Z[k] in X[k] on entry (k < K); thread k <= K/2
@@ -272,12 +300,13 @@ static int exec_c2c(cufftHandle h, const float2* in, float2* out, int dir) {
 // Lay out a length's tables on stream st (l.mem of l.bytes bytes allocated).
 static int fill_length(R2CEngine& e, R2CLength& l, long long K, int S, int nq, int shift, cudaStream_t st) {
     float4* tab = static_cast<float4*>(l.mem);
-    l.ph = Phase{tab, (unsigned)S, (unsigned)shift};
-    k_phase_tables<<<(S + nq + 255) / 256, 256, 0, st>>>(tab, K, S, nq);
+    double2* dbl = reinterpret_cast<double2*>(tab + S + nq);
+    l.ph = Phase{tab, dbl, (unsigned)S, (unsigned)shift};
+    k_phase_tables<<<(S + nq + 255) / 256, 256, 0, st>>>(tab, dbl, K, S, nq);
     if (cudaGetLastError() != cudaSuccess) return -1;
     const long long P = bluestein_points(K);
     if (!P) return 0;
-    l.w = reinterpret_cast<float2*>(tab + S + nq);
+    l.w = reinterpret_cast<float2*>(dbl + S + nq);
     l.fb = l.w + K + (K & 1);
     cufftHandle h;
     if (c2c_plan(e, P, &h) || cufftSetStream(h, st) != CUFFT_SUCCESS) return -1;
@@ -324,7 +353,7 @@ static int length_entry(R2CEngine& e, long long K, cudaStream_t st, R2CLength** 
     const int S = 1 << shift, nq = (int)((2 * K + S - 1) / S);
     const long long P = bluestein_points(K);
     R2CLength* l = new R2CLength;
-    l->bytes = sizeof(float4) * (size_t)(S + nq) + (P ? sizeof(float2) * (size_t)(K + (K & 1) + P) : 0);
+    l->bytes = (sizeof(float4) + sizeof(double2)) * (size_t)(S + nq) + (P ? sizeof(float2) * (size_t)(K + (K & 1) + P) : 0);
     while (!e.lengths.empty() && e.length_bytes + l->bytes > kLengthBytes) {
         auto lru = e.lengths.begin();
         for (auto i = e.lengths.begin(); i != e.lengths.end(); ++i)
