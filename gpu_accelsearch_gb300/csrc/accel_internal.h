@@ -224,8 +224,8 @@ struct RefineNodes {
     double x[kRefineNodes / 2], w[kRefineNodes / 2];
 };
 int refine_panels(double z, double zreach);
-// Widest window (panels) the node rule takes; a call with a wider one runs
-// the direct form, whose work grows with the width and not its square.
+// Widest window (panels) the node rule takes; a candidate with a wider one
+// takes the direct form, whose work grows with the width and not its square.
 // Measured on one candidate of one harmonic, node rule against direct: z =
 // 200 0.25 / 2.9 ms, 1000 1.4 / 13, 3000 9.7 / 39, 5000 26 / 64 (217
 // panels); the lines meet near z = 12000 and the limit is z = 8900, above

@@ -32,7 +32,12 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
     if (rc) return rc;
     std::vector<OptCand> cand((size_t)n);
     const double zreach = refine ? 2.63 : 0.0;  // how far the grids reach in z
-    int maxharm = 1, maxdata = 1, maxpanels = 0;
+    int maxharm = 1, maxdata = 1;
+    // the candidates in launch order: those whose windows suit the node rule,
+    // then the wider ones, for the direct form.  Each goes by its own width,
+    // so that what else is in the list changes neither its result nor its cost.
+    std::vector<long long> order, wide;
+    order.reserve((size_t)n);
     for (long long i = 0; i < n; i++) {
         const accel_candidate& x = in[i];
         if (x.trial < 0 || x.trial >= ntrials || x.numharm < 1 || x.numharm > c->nh ||
@@ -44,6 +49,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         o.numharm = x.numharm;
         o.trial = x.trial;
         maxharm = std::max(maxharm, x.numharm);
+        int maxpanels = 0;
         // harmonic k of H is the bank's harmonic p/q = k/H in lowest terms;
         // its segment in the candidate's step is the search's (A6/A7)
         const long long startr = rlo[x.trial] + (long long)x.step * (c->uselen / 2);
@@ -59,22 +65,27 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
             o.panels[k - 1] = refine_panels(x.z * k / x.numharm, zreach * k / x.numharm);
             maxpanels = std::max(maxpanels, o.panels[k - 1]);
         }
+        (maxpanels > kRefineMaxPanels ? wide : order).push_back(i);
     }
+    const long long nnear = (long long)order.size();
+    order.insert(order.end(), wide.begin(), wide.end());
     if (n == 0) return ACCEL_OK;
     // launches of at most kOptBatch candidates and kOptNodes nodes, from one
     // workspace kept by the context: spectra table, candidates, results,
     // norms and node values
     constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 21;
-    const bool direct = maxpanels > kRefineMaxPanels;
     long long most = 0, most_nodes = 0;
     std::vector<long long> ends;  // end of each launch's candidates
     for (long long i = 0; i < n;) {
+        const bool direct = i >= nnear;
+        const long long end = std::min(direct ? n : nnear, i + kOptBatch);
         long long nodes = 0, j = i;
-        for (; j < n && j - i < kOptBatch; j++) {
+        for (; j < end; j++) {
+            OptCand& o = cand[order[j]];
             long long own = 0;
-            for (int k = 0; k < cand[j].numharm && !direct; k++) own += (long long)cand[j].panels[k] * kRefineNodes;
+            for (int k = 0; k < o.numharm && !direct; k++) own += (long long)o.panels[k] * kRefineNodes;
             if (j > i && nodes + own > kOptNodes) break;
-            cand[j].scratch_off = nodes;
+            o.scratch_off = nodes;
             nodes += own;
         }
         most = std::max(most, j - i);
@@ -114,7 +125,8 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         const long long m = i1 - i0;
         std::memcpy(host, wspec, sizeof(float2*) * ntrials);
         std::memcpy(host + off_nb, numbins, sizeof(long long) * ntrials);
-        std::memcpy(host + off_in, cand.data() + i0, sizeof(OptCand) * m);
+        OptCand* hin = reinterpret_cast<OptCand*>(host + off_in);
+        for (long long j = i0; j < i1; j++) hin[j - i0] = cand[order[j]];
         e = cudaMemcpyAsync(dev, host, off_in + sizeof(OptCand) * m, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) {
             RefineArgs a{};
@@ -129,7 +141,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
             a.refine = refine != 0;
             a.exact_rsqrt = c->cfg.exact_rsqrt;
             a.maxdata = maxdata;
-            if ((direct ? launch_refine_direct(a, c->stream) : launch_refine(a, c->stream)) != 0) {
+            if ((i0 >= nnear ? launch_refine_direct(a, c->stream) : launch_refine(a, c->stream)) != 0) {
                 e = cudaGetLastError();
                 if (e == cudaSuccess) e = cudaErrorUnknown;
             }
@@ -139,7 +151,8 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess)
             return set_error(ACCEL_ERR_CUDA, "accel_optimize_candidates: %s", cudaGetErrorString(e));
-        std::memcpy(res.data() + i0, host + off_out, sizeof(OptOut) * m);
+        const OptOut* hout = reinterpret_cast<const OptOut*>(host + off_out);
+        for (long long j = i0; j < i1; j++) res[order[j]] = hout[j - i0];
         i0 = i1;
     }
     for (long long i = 0; i < n; i++) {
