@@ -457,6 +457,40 @@ int alloc_work(accel_ctx* c) {
     return ACCEL_OK;
 }
 
+// What is only kept for later calls goes back: the transform's tables and
+// working array, the refinement's workspace.  Waits for the context's stream,
+// so that the memory is free when this returns; false when there was nothing,
+// or the stream is being captured.
+static bool give_back(accel_ctx* c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if ((!c->r2c.held() && !c->opt_dev) || cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone)
+        return false;
+    c->r2c.release(c->stream);
+    cudaFree(c->opt_dev);
+    c->opt_dev = nullptr;
+    c->opt_dev_cap = 0;
+    return cudaStreamSynchronize(c->stream) == cudaSuccess;
+}
+
+cudaError_t ctx_malloc(accel_ctx* c, void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // not left for the next launch's check to find
+    return give_back(c) ? cudaMalloc(p, bytes) : e;
+}
+template <class T> static cudaError_t ctx_malloc(accel_ctx* c, T** p, size_t bytes) {
+    return ctx_malloc(c, reinterpret_cast<void**>(p), bytes);
+}
+// The same in stream order on the context's stream.
+template <class T> static cudaError_t ctx_malloc_async(accel_ctx* c, T** p, size_t bytes) {
+    void** v = reinterpret_cast<void**>(p);
+    const cudaError_t e = cudaMallocAsync(v, bytes, c->stream);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    return give_back(c) ? cudaMallocAsync(v, bytes, c->stream) : e;
+}
+
 int ensure_segs(accel_ctx* c, long long n) {
     if (n <= c->segs_cap) return ACCEL_OK;
     if (c->d_segs) cudaFree(c->d_segs);
@@ -464,7 +498,7 @@ int ensure_segs(accel_ctx* c, long long n) {
     c->d_segs = nullptr;
     c->h_segs = nullptr;
     long long cap = std::max(n, 2 * c->segs_cap);
-    CK(cudaMalloc(&c->d_segs, sizeof(SegDesc) * cap));
+    CK(ctx_malloc(c, &c->d_segs, sizeof(SegDesc) * cap));
     CK(cudaMallocHost(&c->h_segs, sizeof(SegDesc) * cap));
     c->segs_cap = cap;
     return ACCEL_OK;
@@ -507,9 +541,9 @@ int whiten_plan(accel_ctx* c, unsigned numbins, WhitenPlanDev** out) {
         l[i] = blocks[i].second;
         w.maxlen = std::max(w.maxlen, l[i]);
     }
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&w.d_start), sizeof(int) * w.nb, c->stream));
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&w.d_len), sizeof(int) * w.nb, c->stream));
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&w.d_med), sizeof(double) * w.nb, c->stream));
+    CK(ctx_malloc_async(c, &w.d_start, sizeof(int) * w.nb));
+    CK(ctx_malloc_async(c, &w.d_len, sizeof(int) * w.nb));
+    CK(ctx_malloc_async(c, &w.d_med, sizeof(double) * w.nb));
     // from pageable memory: staged before the call returns, so the vectors
     // may go out of scope
     CK(cudaMemcpyAsync(w.d_start, s.data(), sizeof(int) * w.nb, cudaMemcpyHostToDevice, c->stream));
@@ -533,7 +567,8 @@ int do_whiten(accel_ctx* c, float2* spec, unsigned numbins) {
 
 int do_rfft(accel_ctx* c, const float* series, long long n, float2* spec) {
     ProfScope ps(c, K_RFFT, 1);
-    const int r = r2c_any(c->r2c, series, n, spec, c->stream);
+    int r = r2c_any(c->r2c, series, n, spec, c->stream);
+    if (r == -2 && c->opt_dev && give_back(c)) r = r2c_any(c->r2c, series, n, spec, c->stream);
     if (r == -2) return set_err(ACCEL_ERR_NOMEM, "real-to-complex transform of %lld samples: scratch memory", n);
     if (r) return set_err(ACCEL_ERR_CUDA, "real-to-complex transform of %lld samples failed", n);
     return ACCEL_OK;
@@ -1281,10 +1316,10 @@ int accel_set_tuning(accel_ctx* c, const accel_tuning* t) {
         c->planes2 = nullptr;
         c->d_step = nullptr;
         c->chunk = t->chunk_segments;
-        CK(cudaMalloc(&c->dbuf, sizeof(float2) * c->dstride * c->chunk));
-        CK(cudaMalloc(&c->planes, sizeof(float) * c->pstride * c->chunk));
-        CK(cudaMalloc(&c->planes2, sizeof(float) * c->pstride * c->chunk));
-        CK(cudaMalloc(&c->d_step, sizeof(unsigned) * ((size_t)c->chunk + 1)));
+        CK(ctx_malloc(c, &c->dbuf, sizeof(float2) * c->dstride * c->chunk));
+        CK(ctx_malloc(c, &c->planes, sizeof(float) * c->pstride * c->chunk));
+        CK(ctx_malloc(c, &c->planes2, sizeof(float) * c->pstride * c->chunk));
+        CK(ctx_malloc(c, &c->d_step, sizeof(unsigned) * ((size_t)c->chunk + 1)));
         encode_hsum_maps(c);
     }
     return ACCEL_OK;
@@ -1437,8 +1472,8 @@ int accel_search(accel_ctx* c, int ntrials, const float* const* series, const lo
             t.series = nullptr;
             t.spec = nullptr;
             t.n = 0;
-            CK(cudaMalloc(&t.series, sizeof(float) * n));
-            CK(cudaMalloc(&t.spec, sizeof(float2) * (n / 2 + 1)));
+            CK(ctx_malloc(c, &t.series, sizeof(float) * n));
+            CK(ctx_malloc(c, &t.spec, sizeof(float2) * (n / 2 + 1)));
             t.n = n;
         }
     }

@@ -39,6 +39,10 @@ struct R2CEngine {
     R2CEngine& operator=(const R2CEngine&) = delete;
     ~R2CEngine();
     void clear();                            // free everything (the stream is idle)
+    // Give back in stream order what is kept for later calls (not the plans):
+    // freed once st has been waited for.
+    void release(cudaStream_t st);
+    size_t held() const { return length_bytes + work_bytes; }
 };
 // spec[0 .. n/2] = the DFT of the n real samples of x (device, n even), on
 // stream st: 0, -1 on a CUDA or cuFFT error, -2 when scratch memory runs out.
@@ -155,6 +159,9 @@ struct accel_ctx {
 namespace accel {
 
 int ensure_device(accel_ctx* c);
+// cudaMalloc for the context; when there is no memory left, once more after
+// giving back what the context only keeps for later calls.
+cudaError_t ctx_malloc(accel_ctx* c, void** p, size_t bytes);
 int ensure_segs(accel_ctx* c, long long n);
 int do_whiten(accel_ctx* c, float2* spec, unsigned numbins);
 int do_rfft(accel_ctx* c, const float* series, long long n, float2* spec);

@@ -72,8 +72,8 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
     if (n == 0) return ACCEL_OK;
     // launches of at most kOptBatch candidates and kOptNodes nodes, from one
     // workspace kept by the context: spectra table, candidates, results,
-    // norms and node values
-    constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 21;
+    // norms and node values (64 MB of those)
+    constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 19;
     long long most = 0, most_nodes = 0;
     std::vector<long long> ends;  // end of each launch's candidates
     for (long long i = 0; i < n;) {
@@ -103,7 +103,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         cudaFree(c->opt_dev);
         c->opt_dev = nullptr;
         c->opt_dev_cap = 0;
-        e = cudaMalloc(&c->opt_dev, dev_bytes);
+        e = ctx_malloc(c, &c->opt_dev, dev_bytes);
         if (e == cudaSuccess) c->opt_dev_cap = dev_bytes;
     }
     if (e == cudaSuccess && host_bytes > c->opt_host_cap) {

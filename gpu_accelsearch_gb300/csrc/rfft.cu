@@ -290,6 +290,13 @@ static long long bluestein_points(long long K) {
     return P;
 }
 
+// Points of the transform's cuFFT plan, 0 where it uses none.
+static long long plan_points(long long K) {
+    if (const long long P = bluestein_points(K)) return P;
+    const long long L = K & -K;
+    return L > 1 || K == 1 ? L : 0;
+}
+
 static int exec_c2c(cufftHandle h, const float2* in, float2* out, int dir) {
     return cufftExecC2C(h, reinterpret_cast<cufftComplex*>(const_cast<float2*>(in)),
                         reinterpret_cast<cufftComplex*>(out), dir) == CUFFT_SUCCESS
@@ -324,16 +331,31 @@ static void drop_length(R2CEngine& e, std::map<long long, R2CLength*>::iterator 
     e.lengths.erase(it);
 }
 
-// Memory in stream order; when there is none, once more after giving back
-// what is kept for other lengths.
-static int alloc_on(R2CEngine& e, void** p, size_t bytes, cudaStream_t st, const R2CLength* in_use) {
-    if (cudaMallocAsync(p, bytes, st) == cudaSuccess) return 0;
-    cudaGetLastError();
+static void drop_work(R2CEngine& e, cudaStream_t st) {
+    if (e.work) cudaFreeAsync(e.work, st);
+    e.work = nullptr;
+    e.work_bytes = 0;
+}
+
+// Everything kept but one length's tables, in stream order.
+static void drop_others(R2CEngine& e, const R2CLength* in_use, cudaStream_t st) {
     for (auto it = e.lengths.begin(); it != e.lengths.end();) {
         auto next = std::next(it);
         if (it->second != in_use) drop_length(e, it, st);
         it = next;
     }
+    drop_work(e, st);
+}
+
+void R2CEngine::release(cudaStream_t st) { drop_others(*this, nullptr, st); }
+
+// Memory in stream order; when there is none, once more after giving back
+// what is kept for other lengths and the working array (not in use while
+// either is allocated).
+static int alloc_on(R2CEngine& e, void** p, size_t bytes, cudaStream_t st, const R2CLength* in_use) {
+    if (cudaMallocAsync(p, bytes, st) == cudaSuccess) return 0;
+    cudaGetLastError();
+    drop_others(e, in_use, st);
     if (cudaMallocAsync(p, bytes, st) == cudaSuccess) return 0;
     cudaGetLastError();
     *p = nullptr;
@@ -354,7 +376,8 @@ static int length_entry(R2CEngine& e, long long K, cudaStream_t st, R2CLength** 
     const long long P = bluestein_points(K);
     R2CLength* l = new R2CLength;
     l->bytes = (sizeof(float4) + sizeof(double2)) * (size_t)(S + nq) + (P ? sizeof(float2) * (size_t)(K + (K & 1) + P) : 0);
-    while (!e.lengths.empty() && e.length_bytes + l->bytes > kLengthBytes) {
+    // (a length too large to keep leaves again after the call)
+    while (l->bytes <= kLengthBytes && e.length_bytes + l->bytes > kLengthBytes) {
         auto lru = e.lengths.begin();
         for (auto i = e.lengths.begin(); i != e.lengths.end(); ++i)
             if (i->second->last_use < lru->second->last_use) lru = i;
@@ -436,14 +459,23 @@ int r2c_any(R2CEngine& e, const float* x, long long n, float2* out, cudaStream_t
     R2CEngine once;
     R2CEngine& owner = keep ? e : once;
     if (!keep) once.plans.swap(e.plans);  // plans are used either way
+    // the plan first: when its work area finds no memory, once more after
+    // giving back (and waiting: the plan's memory is not stream-ordered) what
+    // is kept, of which nothing is in use yet
     R2CLength* l = nullptr;
-    int rc = length_entry(owner, K, st, &l);
+    cufftHandle h;
+    int rc = plan_points(K) ? c2c_plan(owner, plan_points(K), &h) : 0;
+    if (rc && keep && e.held()) {
+        cudaGetLastError();
+        e.release(st);
+        cudaStreamSynchronize(st);
+        rc = c2c_plan(e, plan_points(K), &h);
+    }
+    if (!rc) rc = length_entry(owner, K, st, &l);
     void* work = nullptr;
     if (!rc && wbytes) {
         if (owner.work_bytes < wbytes) {
-            if (owner.work) cudaFreeAsync(owner.work, st);
-            owner.work = nullptr;
-            owner.work_bytes = 0;
+            drop_work(owner, st);
             rc = alloc_on(owner, &owner.work, wbytes, st, l);
             if (!rc) owner.work_bytes = wbytes;
         }
@@ -460,17 +492,10 @@ int r2c_any(R2CEngine& e, const float* x, long long n, float2* out, cudaStream_t
         if (!rc) rc = r2c_with(owner, *l, z, K, out, w, st);
     }
     // a length or working array too large to keep
-    if (keep && !rc && l->bytes > kLengthBytes) drop_length(e, e.lengths.find(K), st);
-    if (keep && e.work_bytes > kLengthBytes) {
-        cudaFreeAsync(e.work, st);
-        e.work = nullptr;
-        e.work_bytes = 0;
-    }
+    if (keep && l && l->bytes > kLengthBytes) drop_length(e, e.lengths.find(K), st);
+    if (keep && e.work_bytes > kLengthBytes) drop_work(e, st);
     if (!keep) {
-        while (!once.lengths.empty()) drop_length(once, once.lengths.begin(), st);
-        if (once.work) cudaFreeAsync(once.work, st);
-        once.work = nullptr;
-        once.work_bytes = 0;
+        once.release(st);
         e.plans.swap(once.plans);
     }
     return rc;

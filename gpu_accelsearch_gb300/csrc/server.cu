@@ -121,6 +121,7 @@ struct accel_server {
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};    // each buffer's last DMA
     bool stage_used[2] = {false, false};
     accel_ctx* wctx = nullptr;       // R2C engine and whitening plans of the admission thread
+    std::mutex prep_mu;              // held while wctx is used (the scheduler takes its memory back at need)
     std::thread worker, admitter;
     bool admitter_done = false;
     std::deque<Request*> ready;      // admitted and prepared, not yet with the scheduler
@@ -204,6 +205,29 @@ void free_group(Group& g) {
     g.ctx = nullptr;
 }
 
+// The tables that the transform keeps per length count against the budget:
+// they go back (in stream order) when they and the admitted requests exceed
+// it together.  prep_mu is held.
+void fit_budget(accel_server* s) {
+    const double held = (double)s->wctx->r2c.held();
+    bool over;
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        over = s->bytes_in_use + held > s->cfg.hbm_budget_bytes;
+    }
+    if (over) s->wctx->r2c.release(s->astream);
+}
+
+// All of them, for an allocation that found no memory; false when none were
+// kept.
+bool take_back(accel_server* s) {
+    std::lock_guard<std::mutex> lk(s->prep_mu);
+    if (!s->wctx->r2c.held()) return false;
+    cudaGetLastError();
+    s->wctx->r2c.release(s->astream);
+    return cudaStreamSynchronize(s->astream) == cudaSuccess;
+}
+
 accel_ctx* group_ctx(accel_server* s, int zmax, int* rc) {
     Group& g = s->groups[zmax];
     if (g.ctx) return g.ctx;
@@ -216,6 +240,7 @@ accel_ctx* group_ctx(accel_server* s, int zmax, int* rc) {
     cfg.chunk_segments = std::max(s->cfg.chunk_segments, s->cfg.max_chunk_segments);
     cfg.device = s->cfg.device;
     *rc = accel_create(&cfg, &g.ctx);
+    if (*rc && *rc != ACCEL_ERR_INVALID && take_back(s)) *rc = accel_create(&cfg, &g.ctx);
     if (*rc) {
         g.ctx = nullptr;
         return nullptr;
@@ -248,8 +273,11 @@ accel_ctx* group_ctx(accel_server* s, int zmax, int* rc) {
 // admission stream), then record its event.
 int admit(accel_server* s, Request* r) {
     int rc = ACCEL_OK;
-    if (cudaMallocAsync(&r->d_series, sizeof(float) * r->n, s->astream) != cudaSuccess ||
-        cudaMallocAsync(&r->d_spec, sizeof(float2) * (r->n / 2 + 1), s->astream) != cudaSuccess)
+    auto alloc = [&](auto** p, size_t bytes) {
+        return cudaMallocAsync(p, bytes, s->astream) == cudaSuccess ||
+               (take_back(s) && cudaMallocAsync(p, bytes, s->astream) == cudaSuccess);
+    };
+    if (!alloc(&r->d_series, sizeof(float) * r->n) || !alloc(&r->d_spec, sizeof(float2) * (r->n / 2 + 1)))
         return set_error(ACCEL_ERR_NOMEM, "request %lld: device allocation", r->id);
     if (s->stage[0] && s->stage[1]) {
         int k = 0;
@@ -273,7 +301,10 @@ int admit(accel_server* s, Request* r) {
     if (cudaEventCreate(&r->ev_prep) != cudaSuccess || cudaEventCreate(&r->ready) != cudaSuccess ||
         cudaEventRecord(r->ev_prep, s->astream) != cudaSuccess)
         return set_error(ACCEL_ERR_CUDA, "request %lld: event", r->id);
+    std::lock_guard<std::mutex> prep(s->prep_mu);
+    fit_budget(s);
     rc = do_rfft(s->wctx, r->d_series, r->n, r->d_spec);
+    fit_budget(s);
     if (!rc) rc = do_whiten(s->wctx, r->d_spec, (unsigned)r->numbins);
     if (!rc && cudaEventRecord(r->ready, s->astream) != cudaSuccess)
         rc = set_error(ACCEL_ERR_CUDA, "request %lld: event", r->id);

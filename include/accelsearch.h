@@ -148,6 +148,13 @@ typedef struct accel_tuning {
                             /* stays usable                                   */
 } accel_tuning;
 
+/* Besides what its plan needs (template bank, planes, candidate buffer), a
+ * context keeps device memory of its calls for the next ones until it is
+ * destroyed: the trials' series and spectra, whitening plans of the last 64
+ * lengths, the transform's tables per length and its working array (each at
+ * most 512 MB, the least recently used lengths leaving) and the refinement's
+ * workspace (about 100 MB at most).  The last three go back by themselves
+ * when an allocation of the context finds no memory. */
 typedef struct accel_ctx accel_ctx;
 
 /* ---------------------------------------------------------------- context */
@@ -322,7 +329,8 @@ int  accel_bank_spectra(const accel_ctx *ctx, int h, accel_complex *kstd, accel_
  * reference, whose driver searches one trial per process run).  An
  * admission thread admits requests in arrival order while their device
  * memory (series and spectrum, 12 bytes per sample) fits
- * hbm_budget_bytes, and copies, transforms and whitens them on its own
+ * hbm_budget_bytes (the transform's tables, kept per length, count too and
+ * go back when there is no room beside the requests), and copies, transforms and whitens them on its own
  * stream; a scheduler thread fills each launch group from one template
  * bank (one bank per zmax, built on first use), shortest remaining work
  * first -- a request admitted while others are in flight joins the next
