@@ -354,13 +354,13 @@ __device__ __forceinline__ uint32_t block_select_reg(const uint32_t (&key)[NK], 
         s = s >= 2 ? s - 2 : 0;
     }
     // one key left in [lo, lo + 2^s)
-    uint32_t mine = 0;
+    uint32_t mine = kNone;
 #pragma unroll
     for (int j = 0; j < NK; j++)
-        if (key[j] - lo < (1u << s)) mine = key[j];
-    mine = __reduce_or_sync(kNone, mine);
+        if (key[j] - lo < (1u << s)) mine = min(mine, key[j]);
+    mine = __reduce_min_sync(kNone, mine);
     if constexpr (W > 1) {
-        if (mine && lane == 0) scratch[64] = mine;
+        if (mine != kNone && lane == 0) scratch[64] = mine;
         __syncthreads();
         mine = (uint32_t)scratch[64];
     }
