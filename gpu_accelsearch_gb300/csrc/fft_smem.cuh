@@ -122,18 +122,6 @@ template <int DIR, bool PK> __device__ __forceinline__ void dft4(float2* v) {
     v[3] = csub(d02, d13);
 }
 
-// W8^k for direction DIR, k = 1,3 (k=2 is DIR*i)
-template <int DIR> __device__ __forceinline__ float2 w8_1(float2 a) {
-    const float s = 0.70710678118654752440f;  // (1 + DIR i)/sqrt2
-    return DIR > 0 ? make_float2(s * (a.x - a.y), s * (a.x + a.y))
-                   : make_float2(s * (a.x + a.y), s * (a.y - a.x));
-}
-template <int DIR> __device__ __forceinline__ float2 w8_3(float2 a) {
-    const float s = 0.70710678118654752440f;  // (-1 + DIR i)/sqrt2
-    return DIR > 0 ? make_float2(-s * (a.x + a.y), s * (a.x - a.y))
-                   : make_float2(s * (a.y - a.x), -s * (a.x + a.y));
-}
-
 __device__ __forceinline__ float2 cfma(float s, float2 a, float2 b) {  // s a + b
     return make_float2(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y));
 }
