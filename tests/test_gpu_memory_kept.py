@@ -109,6 +109,38 @@ def test_given_back_when_memory_runs_out():
             torch.cuda.empty_cache()
 
 
+def test_new_length_when_memory_runs_out():
+    # the tables of a new length (100 MB) take the place of the others'
+    from gpu_accelsearch_gb300.search import AccelSearch
+    torch.manual_seed(7)
+    xs = [torch.randn(2 * k, device="cuda") for k in (4194301, 4194287, 4194277, 4194271)]
+    with AccelSearch(zmax=0, numharm=1, fftlen=128) as s:
+        want = transform(s, xs[0])
+        for x in xs[1:3]:
+            transform(s, x)
+    with AccelSearch(zmax=0, numharm=1, fftlen=128) as s:
+        for x in xs[1:]:
+            transform(s, x)
+        held = pool_used()
+        spec = torch.empty(xs[0].numel() + 2, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        fill = []
+        try:
+            free = torch.cuda.mem_get_info()[0] - 48 * MB
+            while free > 64 * MB:
+                step = min(free, 32 << 30)
+                fill.append(torch.empty(step // 4, device="cuda"))
+                free -= step
+            s.rfft(xs[0].data_ptr(), xs[0].numel(), spec.data_ptr())
+            s.synchronize()
+            assert torch.equal(spec, want)
+            assert pool_used() <= held
+        finally:
+            fill.clear()
+            torch.cuda.empty_cache()
+
+
 def test_server_counts_it_against_its_budget():
     from gpu_accelsearch_gb300.serving import Server
     rng = np.random.default_rng(8)
