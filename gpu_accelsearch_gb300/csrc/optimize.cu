@@ -36,8 +36,8 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
     // the candidates in launch order: those whose windows suit the node rule,
     // then the wider ones, for the direct form.  Each goes by its own width,
     // so that what else is in the list changes neither its result nor its cost.
+    // (empty without wide ones: as given)
     std::vector<long long> order, wide;
-    order.reserve((size_t)n);
     for (long long i = 0; i < n; i++) {
         const accel_candidate& x = in[i];
         if (x.trial < 0 || x.trial >= ntrials || x.numharm < 1 || x.numharm > c->nh ||
@@ -65,15 +65,23 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
             o.panels[k - 1] = refine_panels(x.z * k / x.numharm, zreach * k / x.numharm);
             maxpanels = std::max(maxpanels, o.panels[k - 1]);
         }
-        (maxpanels > kRefineMaxPanels ? wide : order).push_back(i);
+        if (maxpanels > kRefineMaxPanels) wide.push_back(i);
     }
-    const long long nnear = (long long)order.size();
-    order.insert(order.end(), wide.begin(), wide.end());
     if (n == 0) return ACCEL_OK;
+    const long long nnear = n - (long long)wide.size();
+    if (!wide.empty()) {
+        for (long long i = 0, w = 0; i < n; i++) {
+            if (w < (long long)wide.size() && wide[w] == i) w++;
+            else order.push_back(i);
+        }
+        order.insert(order.end(), wide.begin(), wide.end());
+    }
+    auto at = [&](long long j) { return order.empty() ? j : order[j]; };
     // launches of at most kOptBatch candidates and kOptNodes nodes, from one
     // workspace kept by the context: spectra table, candidates, results,
-    // norms and node values (64 MB of those)
-    constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 19;
+    // norms and node values (256 MB of those; with 64 MB a list of 1000
+    // candidates took 7.6 ms instead of 7.4: more launches end in a part wave)
+    constexpr long long kOptBatch = 1 << 16, kOptNodes = 1LL << 21;
     long long most = 0, most_nodes = 0;
     std::vector<long long> ends;  // end of each launch's candidates
     for (long long i = 0; i < n;) {
@@ -81,7 +89,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         const long long end = std::min(direct ? n : nnear, i + kOptBatch);
         long long nodes = 0, j = i;
         for (; j < end; j++) {
-            OptCand& o = cand[order[j]];
+            OptCand& o = cand[at(j)];
             long long own = 0;
             for (int k = 0; k < o.numharm && !direct; k++) own += (long long)o.panels[k] * kRefineNodes;
             if (j > i && nodes + own > kOptNodes) break;
@@ -126,7 +134,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         std::memcpy(host, wspec, sizeof(float2*) * ntrials);
         std::memcpy(host + off_nb, numbins, sizeof(long long) * ntrials);
         OptCand* hin = reinterpret_cast<OptCand*>(host + off_in);
-        for (long long j = i0; j < i1; j++) hin[j - i0] = cand[order[j]];
+        for (long long j = i0; j < i1; j++) hin[j - i0] = cand[at(j)];
         e = cudaMemcpyAsync(dev, host, off_in + sizeof(OptCand) * m, cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) {
             RefineArgs a{};
@@ -152,7 +160,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
         if (e != cudaSuccess)
             return set_error(ACCEL_ERR_CUDA, "accel_optimize_candidates: %s", cudaGetErrorString(e));
         const OptOut* hout = reinterpret_cast<const OptOut*>(host + off_out);
-        for (long long j = i0; j < i1; j++) res[order[j]] = hout[j - i0];
+        for (long long j = i0; j < i1; j++) res[at(j)] = hout[j - i0];
         i0 = i1;
     }
     for (long long i = 0; i < n; i++) {

@@ -153,7 +153,7 @@ typedef struct accel_tuning {
  * destroyed: the trials' series and spectra, whitening plans of the last 64
  * lengths, the transform's tables per length and its working array (each at
  * most 512 MB, the least recently used lengths leaving) and the refinement's
- * workspace (about 100 MB at most).  The last three go back by themselves
+ * workspace (about 300 MB at most).  The last three go back by themselves
  * when an allocation of the context finds no memory. */
 typedef struct accel_ctx accel_ctx;
 
