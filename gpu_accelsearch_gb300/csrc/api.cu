@@ -66,7 +66,7 @@ double log_gamma_q(int n, double x) {  // log P(Gamma(n,1) > x)
     return -x + std::log(s);
 }
 double log_gauss_tail(double sigma) {  // log P(N(0,1) > sigma)
-    if (sigma < 30.0) return std::log(0.5 * std::erfc(sigma / std::sqrt(2.0)));
+    if (sigma < 30.0) return std::log(0.5 * std::erfc(sigma * M_SQRT1_2));
     // asymptotic expansion beyond double erfc's range
     double s2 = sigma * sigma;
     return -0.5 * s2 - std::log(sigma * std::sqrt(2.0 * M_PI)) + std::log1p(-1.0 / s2 + 3.0 / (s2 * s2));
@@ -102,7 +102,7 @@ double sigma_of_power(double power, int numharm, double numindep) {
         const double lq = log_gauss_tail(s), f = lq - logp;
         const double m = std::exp(-0.5 * s * s - kHalfLog2Pi - lq);
         const double newton = f / m, d = m - s;
-        const double curve = 1.0 + newton * (d + newton * (d * (d + m) - 1.0) / 6.0);
+        const double curve = 1.0 + newton * (d + newton * (d * (d + m) - 1.0) * (1.0 / 6.0));
         const double step = curve > 0.5 ? newton * (1.0 + 0.5 * newton * d) / curve : newton;
         s += step;
         if (s < 0.0) s = 0.0;
