@@ -31,8 +31,9 @@ constexpr int kTwN = 8192;          // twiddle table length (max FFT points)
 // that the threads of a warp fetch theirs by 16-byte loads of consecutive
 // memory (with the four side by side, 32 bytes apart, each such load took 16
 // wavefronts of the L1 data pipe instead of 4, and it is this pipe that the
-// plane kernels fill: 92 % at 2048 points).  Sections: NR = 64, 128, 256 (16
-// entries each), 512, 1024, 2048, 4096 (256 entries each).
+// plane kernels fill: 92 % at 2048 points then, 84 % since their rows leave by
+// bulk copies).  Sections: NR = 64, 128, 256 (16 entries each), 512, 1024,
+// 2048, 4096 (256 entries each).
 ACCEL_HD constexpr int tw_pack_entries(int NR) { return NR <= 256 ? 16 : 256; }
 ACCEL_HD constexpr int tw_pack_off(int NR) {  // in float2, from the start of the packed part
     return NR == 64 ? 0 : NR == 128 ? 64 : NR == 256 ? 128 : NR == 512 ? 192 : NR == 1024 ? 1216

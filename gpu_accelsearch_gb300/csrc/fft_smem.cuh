@@ -72,8 +72,10 @@ template <int M> struct FftShape {
 // instruction (add/sub/fma.rn.f32x2, the same roundings as two).  A packed
 // instruction holds the FP32 pipe as long as two, so what it saves is issue
 // slots: 54 -> 45 instructions per point, which moves the plane kernels 2 to 3
-// % (their L1 data pipe is the busier unit).  The 8192-point transform (one
-// CTA of 16 warps per SM) is 3 % slower packed and keeps the scalar forms.
+// % (their L1 data pipe is the busier unit).  The 8192-point transform keeps the
+// scalar forms: both transforms of a row in one CTA, 16 warps and nothing else
+// on the SM, measured 3 % slower packed (that form serves options only now; the
+// default k_plane_half took the scalar sums over and was not measured packed).
 template <bool PK> __device__ __forceinline__ float2 padd(float2 a, float2 b) {
     if constexpr (!PK) return cadd(a, b);
     float2 r;

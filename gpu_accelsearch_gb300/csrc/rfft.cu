@@ -12,18 +12,17 @@
 //     Z[k] = conj(w[k]) sum_n (z[n] conj(w[n])) w[k - n],
 // a linear convolution done by power-of-two transforms of P >= 2K - 1
 // points.  Every phase is a multiple of pi/K reduced exactly to r in
-// [0, 2K) (m^2 mod 2K in integers) and evaluated as the product of two table
-// entries, exp(i pi q S/K) exp(i pi t/K) with r = q S + t, S ~ sqrt(2K),
-// and gives the double-precision product of the two rounded once to float.
-// The double-precision operations (1/64 of the FP32 rate: the four per bin
-// alone held the unpacking kernel at 15 us for K = 2^21, now 8.5) are done only
-// where they can matter: the entries are kept as sums of two floats as well,
-// multiplied with the products' rounding errors carried along, and only where
-// that result lies so close to the middle of two floats that its own error
-// could decide (3 in 100000) is the double product formed.  The N/2 + 1 bins
-// follow from the
-// transforms of the even and odd samples, E[k] = (Z[k] + conj Z[K-k]) / 2
-// and O[k] = (Z[k] - conj Z[K-k]) / (2i):
+// [0, 2K) (m^2 mod 2K in integers) and evaluated as the double-precision
+// product of two table entries, exp(i pi q S/K) exp(i pi t/K) with r = q S + t,
+// S ~ sqrt(2K), rounded once to float.  The double-precision operations (1/64
+// of the FP32 rate: the four per bin alone held the unpacking kernel at 15 us
+// for K = 2^21, now 9) are done only where they can matter: the entries are
+// kept as sums of two floats as well, multiplied with the products' rounding
+// errors carried along, and only where that result lies so close to the middle
+// of two floats that its own error could decide (3 in 100000) is the double
+// product formed.  The N/2 + 1 bins follow from the transforms of the even and
+// odd samples, E[k] = (Z[k] + conj Z[K-k]) / 2 and O[k] = (Z[k] - conj Z[K-k])
+// / (2i):
 //     X[k] = E[k] + exp(-2 pi i k / N) O[k],   k = 0 .. K   (Z[K] = Z[0]).
 // A plan per power of two serves every length, so a stream of trials of
 // many lengths (the serving path) makes no new cuFFT plan per trial --
@@ -34,7 +33,8 @@
 // and the transform of its wrapped filter -- is laid out once per length and
 // kept with the plans (the DM trials of an observation share one length),
 // least recently used lengths leaving when more than kLengthBytes are held;
-// the working arrays are kept too.  A call of Bluestein's form is then two
+// the working arrays are kept too, and all of it goes back when an allocation
+// of the context finds no memory (R2CEngine::release).  A call of Bluestein's form is then two
 // power-of-two transforms instead of three, and at 2 x 609997 samples
 // 74 us of kernels instead of 126 (cold cache).
 #include <algorithm>

@@ -179,13 +179,14 @@ __device__ __forceinline__ float* stage_row_powers(const HarmPlan& H, unsigned c
 
 // Rows gathered in shared memory and stored by one bulk copy each, instead of
 // 8-byte stores from the registers.  A store of 256 bytes by a warp takes 6.6
-// wavefronts of the L1 data pipe, a fifth of a 2048-point row's, and the pipe
-// is 92 % busy there; through shared memory the row costs 2 wavefronts for the
-// same bytes, one more barrier pair and the wait of one thread for the copy's
-// reads.  us per segment, stores -> bulk: 2048 points 4.43 -> 4.30 (656 rows),
-// 1024 1.31 -> 1.27, 512 0.64 -> 0.64 (400 rows).  At 4096 points the pipe is
-// 70 % busy and two CTAs per SM hide the wait less: 10.39 -> 10.42.  A buffer of its own for the row saves a barrier but
-// takes the L1's room: 4.79.
+// wavefronts of the L1 data pipe, a fifth of a 2048-point row's, and with such
+// stores the pipe was 92 % busy there (84 % now); through shared memory the row
+// costs 2 wavefronts for the same bytes, one more barrier pair and the wait of
+// one thread for the copy's reads.  us per segment, stores -> bulk: 2048 points
+// 4.43 -> 4.30 (656 rows), 1024 1.31 -> 1.27, 512 0.64 -> 0.64 (400 rows).  At
+// 4096 points the pipe is 70 % busy and two CTAs per SM hide the wait less:
+// 10.39 -> 10.42.  A buffer of its own for the row saves a barrier but takes
+// the L1's room: 4.79.
 constexpr bool plane_bulk_rows(int M) { return M == 1024 || M == 2048; }
 
 template <int M, bool F16, bool SPLIT>
@@ -284,7 +285,7 @@ struct PlaneHalf {
 template <bool F16>
 __global__ void __launch_bounds__(PlaneHalf::THREADS, 2) k_plane_half(const PlaneArgs a, const float2* __restrict__ tw) {
     constexpr int M = PlaneHalf::M, T = PlaneHalf::THREADS, PITCH = PlaneHalf::PITCH;
-    constexpr bool PK = M < 8192;  // as fft_smem.cuh's transform
+    constexpr bool PK = M < 8192;  // as fft_smem.cuh's transform (packed not measured in this form)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
     const int item = blockIdx.y;
