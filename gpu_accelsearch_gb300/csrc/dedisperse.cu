@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "../../include/accelsearch.h"
@@ -258,57 +259,94 @@ __global__ void __launch_bounds__(kDdThreads, 2)
     }
 }
 
-// Tables of the windowed form for tiles of D trials; false where the offsets
-// of some tile do not fit (spread in samples, or the ring in shared memory).
+// Tables of the windowed form: window starts [ndtile][nchan], then (16-byte
+// aligned) the trials' byte offsets [ndtile][whole stages of channels][D].
+// Filling them is the call's host work, and with many trials of short outputs
+// most of its time: every loop below runs along the channels.  (1024 channels x
+// 2048 trials x 4096 samples 3.8 ms; with a pass over the delays for each tile
+// height and the offsets filled down the trials 8.9; with 32-bit delays relative
+// to 16-trial tiles, as the windows were copied sample by sample, 5.7.)
 struct DwPlan {
     int ndtile = 0, wlen = 0;
-    std::vector<long long> start;
-    std::vector<unsigned short> offs;
+    size_t offs_at = 0, bytes = 0;
+    std::unique_ptr<char[]> tab;
 };
 
 static size_t dw_smem(int D, int wlen) { return sizeof(float) * kDwS * kDwC * (size_t)wlen + 2 * kDwS * kDwC * D; }
 
-// Widest delay range of a channel within a tile of D trials.
-static int dw_spread(const int* delays, int nchan, int ndm, int D) {
-    int spread = 0;
-    std::vector<int> lo(nchan), hi(nchan);
-    for (int d0 = 0; d0 < ndm; d0 += D) {
-        const int n = std::min(D, ndm - d0);
-        const int* first = delays + (long long)d0 * nchan;
-        std::copy(first, first + nchan, lo.begin());
-        std::copy(first, first + nchan, hi.begin());
-        for (int j = 1; j < n; j++) {
-            const int* row = first + (long long)j * nchan;
-            for (int c = 0; c < nchan; c++) {
-                lo[c] = std::min(lo[c], row[c]);
-                hi[c] = std::max(hi[c], row[c]);
+// Smallest and largest delay of every channel over tiles of 4, 8 and 16 trials.
+struct DwBounds {
+    std::vector<int> lo[3], hi[3];  // [tile][nchan]
+    int spread[3];                  // widest range of a channel within a tile
+};
+
+static void dw_bounds(DwBounds& b, const int* delays, int nchan, int ndm) {
+    for (int k = 0; k < 3; k++) {
+        const int D = 4 << k, nt = (ndm + D - 1) / D, parts = k ? (ndm + D / 2 - 1) / (D / 2) : ndm, per = k ? 2 : 4;
+        const int* lo_in = k ? b.lo[k - 1].data() : delays;
+        const int* hi_in = k ? b.hi[k - 1].data() : delays;
+        b.lo[k].resize((size_t)nt * nchan);
+        b.hi[k].resize((size_t)nt * nchan);
+        int spread = 0;
+        for (int t = 0; t < nt; t++) {
+            int* lo = b.lo[k].data() + (size_t)t * nchan;
+            int* hi = b.hi[k].data() + (size_t)t * nchan;
+            std::copy(lo_in + (size_t)t * per * nchan, lo_in + ((size_t)t * per + 1) * nchan, lo);
+            std::copy(hi_in + (size_t)t * per * nchan, hi_in + ((size_t)t * per + 1) * nchan, hi);
+            for (int j = t * per + 1; j < std::min(parts, (t + 1) * per); j++) {
+                const int* l = lo_in + (size_t)j * nchan;
+                const int* h = hi_in + (size_t)j * nchan;
+                for (int c = 0; c < nchan; c++) {
+                    lo[c] = std::min(lo[c], l[c]);
+                    hi[c] = std::max(hi[c], h[c]);
+                }
             }
+            for (int c = 0; c < nchan; c++) spread = std::max(spread, hi[c] - lo[c]);
         }
-        for (int c = 0; c < nchan; c++) spread = std::max(spread, hi[c] - lo[c]);
+        b.spread[k] = spread;
     }
-    return spread;
 }
 
-static void dw_plan(DwPlan& p, const float* in, const int* delays, int nchan, long long nsamp, int ndm, int D,
-                    int wlen) {
+// k: the tile height is D = 4 << k.
+static void dw_plan(DwPlan& p, const DwBounds& b, const float* in, const int* delays, int nchan, long long nsamp,
+                    int ndm, int k, int wlen) {
+    const int D = 4 << k, Q = D / 4;
     p.ndtile = (ndm + D - 1) / D;
     p.wlen = wlen;
-    p.start.resize((size_t)p.ndtile * nchan);
     const size_t pad = (size_t)(nchan + kDwC - 1) / kDwC * kDwC;  // whole stages: 16-byte rows to copy
-    p.offs.assign(p.ndtile * pad * D, 0);
+    p.offs_at = (sizeof(long long) * p.ndtile * nchan + 15) & ~(size_t)15;
+    p.bytes = p.offs_at + sizeof(unsigned short) * p.ndtile * pad * D;
+    p.tab.reset(new char[p.bytes]);
     const long long skew = (long long)((reinterpret_cast<uintptr_t>(in) >> 2) & 3);
+    std::vector<int> base(nchan);             // sample offset of delay 0 in the window
+    std::vector<unsigned long long> four(nchan);
     for (int tl = 0; tl < p.ndtile; tl++) {
-        const int n = std::min(D, ndm - tl * D);
-        const int* first = delays + (long long)tl * D * nchan;
+        const int* lo = b.lo[k].data() + (size_t)tl * nchan;
+        long long* start = reinterpret_cast<long long*>(p.tab.get()) + (size_t)tl * nchan;
         for (int c = 0; c < nchan; c++) {
-            int lo = first[c];
-            for (int j = 1; j < n; j++) lo = std::min(lo, first[(long long)j * nchan + c]);
-            const long long at = (long long)c * nsamp + lo;
+            const long long at = (long long)c * nsamp + lo[c];
             const int rem = (int)((at + skew) & 3);
-            p.start[(size_t)tl * nchan + c] = at - rem;
-            unsigned short* o = p.offs.data() + (tl * pad + c) * D;
-            for (int j = 0; j < n; j++) o[j] = (unsigned short)(4 * (first[(long long)j * nchan + c] - lo + rem));
+            start[c] = at - rem;
+            base[c] = rem - lo[c];
         }
+        // four trials' 16-bit offsets at a time as one 64-bit word (little-endian)
+        char* row = p.tab.get() + p.offs_at + sizeof(unsigned short) * tl * pad * D;
+        for (int q = 0; q < Q; q++) {
+            const int d0 = tl * D + 4 * q;
+            for (int j = 0; j < 4; j++) {
+                if (d0 + j < ndm) {
+                    const int* dl = delays + (size_t)(d0 + j) * nchan;
+                    for (int c = 0; c < nchan; c++) {
+                        const unsigned long long v = (unsigned)(4 * (dl[c] + base[c]));
+                        four[c] = j ? four[c] | v << (16 * j) : v;
+                    }
+                } else if (j == 0) {
+                    std::fill(four.begin(), four.end(), 0ull);  // padding trials
+                }
+            }
+            for (int c = 0; c < nchan; c++) std::memcpy(row + 8 * ((size_t)c * Q + q), &four[c], 8);
+        }
+        std::memset(row + 8 * (size_t)nchan * Q, 0, 8 * (pad - nchan) * Q);
     }
 }
 
@@ -327,10 +365,9 @@ static cudaError_t dw_launch(const DwPlan& p, const float* in, int nchan, long l
         attr_set(attr, dev);
     }
     const long long ntt = (nout + kDwT - 1) / kDwT;
-    const size_t ob = sizeof(long long) * p.start.size();
     k_dedisperse_win<D><<<(unsigned)(p.ndtile * ntt), kDdThreads, dw_smem(D, p.wlen), st>>>(
         in, nchan, (long long)nchan * nsamp, reinterpret_cast<const long long*>(tab),
-        reinterpret_cast<const unsigned short*>(tab + ((ob + 15) & ~(size_t)15)), ndm, p.ndtile, p.wlen, out, nout,
+        reinterpret_cast<const unsigned short*>(tab + p.offs_at), ndm, p.ndtile, p.wlen, out, nout,
         wait_test ? 16u : 0u);
     return cudaGetLastError();
 }
@@ -344,11 +381,12 @@ static int dedisperse(const float* filterbank_dev, int nchan, long long nsamp, c
     if (!filterbank_dev || !out_dev || !delays || nchan < 1 || ndm < 1 || nsamp < 1 || nout < 1)
         return set_error(ACCEL_ERR_INVALID, "accel_dedisperse: bad argument");
     const long long nd = (long long)ndm * nchan;
-    int mx = 0;
+    int mn = 0, mx = 0;
     for (long long i = 0; i < nd; i++) {
-        if (delays[i] < 0) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse: negative delay");
+        mn = std::min(mn, delays[i]);
         mx = std::max(mx, delays[i]);
     }
+    if (mn < 0) return set_error(ACCEL_ERR_INVALID, "accel_dedisperse: negative delay");
     if (nout > nsamp - mx)
         return set_error(ACCEL_ERR_INVALID, "accel_dedisperse: %lld output samples need %lld input samples, have %lld",
                          nout, nout + mx, nsamp);
@@ -357,26 +395,25 @@ static int dedisperse(const float* filterbank_dev, int nchan, long long nsamp, c
     {
         // windowed kernel: the tile height that pads and copies least among
         // those whose windows fit
-        int D = 0, wlen = 0;
+        DwBounds bounds;
+        dw_bounds(bounds, delays, nchan, ndm);
+        int D = 0, wlen = 0, height = 0;
         double best = 0;
-        for (int d : {16, 8, 4}) {
-            const long long spread = dw_spread(delays, nchan, ndm, d), need = (kDwT + spread + 3 + 3) & ~3LL;
+        for (int k : {2, 1, 0}) {
+            const int d = 4 << k;
+            const long long spread = bounds.spread[k], need = (kDwT + spread + 3 + 3) & ~3LL;
             const long long nt = (ndm + d - 1) / d;
             if (4 * (spread + 3) > 65535 || dw_smem(d, (int)need) > kDwSmemMax || nt * ntt > 0x7fffffffLL) continue;
             const double cost = (double)nt * d * (1.0 + (double)need / ((double)kDwT * d));
-            if (!D || cost < best) D = d, wlen = (int)need, best = cost;
+            if (!D || cost < best) D = d, height = k, wlen = (int)need, best = cost;
         }
         if (D) {
             DwPlan p;
-            dw_plan(p, filterbank_dev, delays, nchan, nsamp, ndm, D, wlen);
-            const size_t ob = (sizeof(long long) * p.start.size() + 15) & ~(size_t)15;
-            std::vector<char> tab(ob + sizeof(unsigned short) * p.offs.size());
-            std::memcpy(tab.data(), p.start.data(), sizeof(long long) * p.start.size());
-            std::memcpy(tab.data() + ob, p.offs.data(), sizeof(unsigned short) * p.offs.size());
+            dw_plan(p, bounds, filterbank_dev, delays, nchan, nsamp, ndm, height, wlen);
             char* d_tab = nullptr;
-            cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d_tab), tab.size(), st);
+            cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d_tab), p.bytes, st);
             // from pageable memory: staged before the call returns
-            if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, p.tab.get(), p.bytes, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess)
                 e = D == 16  ? dw_launch<16>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, wait_test, st)
                     : D == 8 ? dw_launch<8>(p, filterbank_dev, nchan, nsamp, d_tab, ndm, out_dev, nout, wait_test, st)
