@@ -226,11 +226,16 @@ struct RefineNodes {
 int refine_panels(double z, double zreach);
 // Widest window (panels) the node rule takes; a candidate with a wider one
 // takes the direct form, whose work grows with the width and not its square.
-// Measured on one candidate of one harmonic, node rule against direct: z =
-// 200 0.25 / 2.9 ms, 1000 1.4 / 13, 3000 9.7 / 39, 5000 26 / 64 (217
-// panels); the lines meet near z = 12000 and the limit is z = 8900, above
-// every f-dot a bank of 16384-point segments can hold.
-constexpr int kRefineMaxPanels = 384;
+// Each candidate goes by its own width, so that its result does not depend on
+// the list.  Node rule / direct form, ms a call:
+//   grids: 1024 candidates of one harmonic z = 200 5.4 / 24, 1000 41 / 81, 2000
+//   136 / 157, 3000 457 / 234; one candidate 0.17 / 2.9, 0.95 / 13, 2.7 / 26,
+//   9.8 / 39.  100 panels, z = 2070: where long lists break even.
+//   one point: candidates of 8 harmonics, one of them z = 20 0.08 / 0.25, 140
+//   0.14 / 0.30, 200 0.20 / 0.36; 512 of them 0.82 / 0.61, 2.0 / 0.80, 3.1 /
+//   0.96.  7 panels, z = 152: beyond, long lists lose more than short ones gain.
+constexpr int kRefineMaxPanels = 100;
+constexpr int kRefineMaxPanelsPoint = 7;
 
 // ---- launchers (return 0 or -1 after a launch error) ----
 int launch_fund_sum(const FundArgs& a, int nseg, const float2* tw, cudaStream_t st);

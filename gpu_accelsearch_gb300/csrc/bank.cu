@@ -316,7 +316,7 @@ int launch_bank_build(const BankHarmDev* hd_dev, const BankHarmDev* hd_host, int
 // Candidate refinement with the responses evaluated directly, bin by bin:
 // the form for windows so wide that refine.cu's node rule, whose work grows
 // with the square of the width, is no longer the cheaper one
-// (kRefineMaxPanels in accel_internal.h).  Definitions as there.
+// (kRefineMaxPanels and kRefineMaxPanelsPoint in accel_internal.h).  Definitions as there.
 // F(x; z), evaluated directly (the reference's small-offset series
 // corrections are expansions of the same function).
 __device__ double2 response_at(double x, double z) {

@@ -65,7 +65,7 @@ extern "C" int accel_optimize_candidates(accel_ctx* c, int ntrials, const accel_
             o.panels[k - 1] = refine_panels(x.z * k / x.numharm, zreach * k / x.numharm);
             maxpanels = std::max(maxpanels, o.panels[k - 1]);
         }
-        if (maxpanels > kRefineMaxPanels) wide.push_back(i);
+        if (maxpanels > (refine ? kRefineMaxPanels : kRefineMaxPanelsPoint)) wide.push_back(i);
     }
     if (n == 0) return ACCEL_OK;
     const long long nnear = n - (long long)wide.size();

@@ -109,3 +109,17 @@ def test_direct_form(bank):
         assert (b["r"], b["z"]) == (r, z)
         want = summed(row, r, z)
         assert np.allclose(b["harm_power"][:H], want, rtol=3e-7) and np.isclose(b["power"], sum(want), rtol=3e-7)
+
+
+# widths on either side of the two forms' limits (z about 152 for one point,
+# 2070 with the grids) and of the window that is staged in shared memory
+@pytest.mark.parametrize("refine", [False, True])
+@pytest.mark.parametrize("z", [140.0, 150.0, 153.0, 156.0, 160.0, 1900.0, 2040.0, 2065.0, 2075.0, 2100.0, 2700.0])
+def test_either_side_of_the_limits(bank, z, refine):
+    s, spec, sp = bank
+    rows = [(1, 30000.3, z, 1), (2, 41000.5, -z, 2)]
+    for (step, r, zz, H), o in zip(rows, s.optimize(cands(rows), RLO, TOBS, spectra=sp, refine=refine)):
+        assert abs(o["r"] - r) <= 0.65626 * refine and abs(o["z"] - zz) <= 2.6251 * refine
+        n2 = O.step_norms(spec, ZMAX, NH, s.uselen, RLO, step, H)
+        want = [n2[k - 1] * power(spec, o["r"] * k / H, o["z"] * k / H) for k in range(1, H + 1)]
+        assert np.allclose(o["harm_power"][:H], want, rtol=3e-7) and np.isclose(o["power"], sum(want), rtol=3e-7)
