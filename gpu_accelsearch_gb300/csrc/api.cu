@@ -579,9 +579,11 @@ int do_rfft(accel_ctx* c, const float* series, long long n, float2* spec) {
 }
 
 // Work of the caller's call is in flight when the call returns: what
-// accel_destroy waits for.  (Work recorded into a caller's graph is the
-// graph's.)
+// accel_destroy waits for -- on the context's own stream by itself, on a
+// caller's, which may be gone by then, by an event.  Work recorded into a
+// caller's graph is the graph's.
 void mark_async(accel_ctx* c) {
+    if (c->own_stream) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
         cudaEventRecord(c->ev_async, c->stream) == cudaSuccess)
@@ -1087,7 +1089,8 @@ void free_ctx(accel_ctx* c) {
     cudaSetDevice(c->device);
     // memory that came from the stream-ordered allocator is freed below
     // without waiting for its users
-    if (c->async_issued) cudaEventSynchronize(c->ev_async);
+    if (c->own_stream) cudaStreamSynchronize(c->stream);
+    else if (c->async_issued) cudaEventSynchronize(c->ev_async);
     c->r2c.clear();
     for (auto& e : c->pending) {
         cudaEventDestroy(e.a);

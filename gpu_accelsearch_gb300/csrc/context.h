@@ -149,9 +149,8 @@ struct accel_ctx {
     std::vector<cudaEvent_t> evpool;
     accel_stats stats{};
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;  // bracket each search call
-    // end of the last transform or whitening issued without waiting for it:
-    // they use memory of the context, which accel_destroy frees (an event,
-    // not the stream: a caller's stream may be gone by then)
+    // end of the last transform or whitening issued on a caller's stream without
+    // waiting for it: they use memory of the context, which accel_destroy frees
     cudaEvent_t ev_async = nullptr;
     bool async_issued = false;
 };
