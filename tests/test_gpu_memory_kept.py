@@ -4,7 +4,7 @@ leaves after its call, everything kept goes back when an allocation finds no
 memory, and in the server it counts against the HBM budget.
 
 What is kept comes from the device's stream-ordered memory pool, whose bytes in
-use and bytes reserved the driver reports (destroying a context leaves the
+use and bytes reserved the CUDA driver reports (destroying a context leaves the
 former as they were: cudaFree of such memory is not counted there)."""
 import ctypes as C
 
